@@ -23,13 +23,15 @@ INCLUDE = PKG.parent / "include"
 LIB = PKG / "libgsw.so"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "--fmad=false", "-lineinfo", "-Xcompiler", "-fPIC",
+# no contraction by the compiler nor by the assembler
+EXACT = ["--fmad=false", "-Xptxas", "--fmad=false"]
+NVCC_FLAGS = ["-O3", "-std=c++17", *EXACT, "-lineinfo", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-fvisibility=hidden", "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr"]
 # The fast-arithmetic compilation of the binary32 step kernels (gsw_fast.cu): FMA
 # contraction and flush-to-zero; its square root and division are the approximate
 # instructions named in gsw_core.cuh.
 FAST_SOURCES = {"gsw_fast.cu"}
-FAST_FLAGS = [f for f in NVCC_FLAGS if f != "--fmad=false"] + ["--fmad=true", "-ftz=true"]
+FAST_FLAGS = ["--fmad=true", "-ftz=true"] + [f for f in NVCC_FLAGS if f not in EXACT]
 
 
 def sources():

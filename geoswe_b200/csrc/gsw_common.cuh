@@ -61,6 +61,19 @@ __device__ __forceinline__ void block_max_to(unsigned long long v, unsigned long
     }
 }
 
+// Max of the warps' wave-speed bits: one atomicMax per warp that exceeds the value it reads.
+// A block-wide reduction would hold the block's finished warps at a barrier until its slowest
+// is done (a tenth of the resident warps' time); the read keeps most warps from the one
+// contended address. Every lane of the warp calls it.
+__device__ __forceinline__ void warp_max_to(unsigned long long v, unsigned long long* target) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+        v = w > v ? w : v;
+    }
+    if (threadIdx.x == 0 && v != 0ull && v > *(volatile unsigned long long*)target) atomicMax(target, v);
+}
+
 // Commit the previous step (t = t_new, steps += 1).
 __device__ __forceinline__ void loop_commit(GswLoopState* s) {
     if (s->pending) {

@@ -15,6 +15,7 @@
 // namespace gsw renamed), so each compilation has its own kernels.
 #pragma once
 #include "gsw_common.cuh"
+#include "gsw_face.cuh"
 
 namespace gsw {
 
@@ -39,6 +40,8 @@ struct DenseK {
     T h_cfl;
     int tile_rows;
     T g_recip;                   // RN(1/g) for the star depth's h / g, or 0 (gsw_core.cuh div_g)
+    bool general;                // binary32: outside face_ranges, every row by the operators
+    bool long_rows;              // binary32: rows too long for 32-bit offsets within a tile
 };
 
 template <typename T>
@@ -94,14 +97,10 @@ __device__ __forceinline__ T dt_of(const GswLoopState* st);
 template <> __device__ __forceinline__ float  dt_of<float>(const GswLoopState* st)  { return st->dt_f32; }
 template <> __device__ __forceinline__ double dt_of<double>(const GswLoopState* st) { return st->dt; }
 
-// STEP = false: residual into o0..o2. STEP = true: updated state into o0..o2.
-// REFPOW: Manning's h^(-4/3) by powf (GSW_ARITH_EXACT) instead of pow_m43.
-// LEAN: the kernel of the production configuration (no inside mask, no CFL skip mask,
-// the wave speed reduced, a Manning class table, quadratic friction, keep-h; rain none
-// or uniform), with those choices compiled in rather than tested per cell: 6 % of the
-// 8192^2 step. Any other configuration takes the general kernel; both give the same bits.
-template <typename T, bool STEP, int MINB, bool REFPOW, bool LEAN>
-__global__ void __launch_bounds__(256, MINB) dense_march_kernel(DenseK<T> p) {
+// Binary64, and binary32 on rows too long for dense_rows_kernel's 32-bit offsets. STEP = false:
+// residual into o0..o2. STEP = true: updated state into o0..o2. REFPOW: as DenseRow's.
+template <typename T, bool STEP, bool REFPOW>
+__global__ void __launch_bounds__(256, 1) dense_march_kernel(DenseK<T> p) {
     if (STEP && p.st->done) return;                       // grid-uniform
     const int lane = threadIdx.x;
     const int strip = blockIdx.x * blockDim.y + threadIdx.y;
@@ -114,7 +113,6 @@ __global__ void __launch_bounds__(256, MINB) dense_march_kernel(DenseK<T> p) {
     const int i0 = p.row_lo + blockIdx.y * p.tile_rows;
     const int i1 = min(i0 + p.tile_rows, p.row_hi);
     unsigned long long lam_local = 0ull;
-    uint32_t lam32 = 0u;        // binary32: the bits of the largest wave speed (lam_dense_bits32)
 
     T dt = (T)0;
     T rate = (T)0;
@@ -149,19 +147,7 @@ __global__ void __launch_bounds__(256, MINB) dense_march_kernel(DenseK<T> p) {
         srm_face<T, true>(cur, nx, p.half_dx, p.inv_dx, p.g, p.h_min, Wf, p.g_recip);
         cur = nx;
 
-#ifdef GSW_FAST_ARITH
-#pragma unroll 2      // two rows in flight: 1.76 -> 1.62 ms at 8192^2 fast (the exact step, and the
-                      // flat march with either arithmetic, slow down)
-#endif
         for (int r = i0; r < i1; ++r) {
-            // the update's class id and running maximum, loaded before the faces so that
-            // their latency is hidden (the production kernel; the general one loads late)
-            uint8_t cls_r = 0;
-            T mh_r = (T)0;
-            if (LEAN && STEP && out_lane) {
-                cls_r = p.ncls[(int64_t)r * p.cpitch + c];
-                if (p.max_h != nullptr) mh_r = p.max_h[(int64_t)r * p.pitch + c];
-            }
             nx.h = pf_h; nx.hu = pf_hu; nx.hv = pf_hv;
             nx.b = b_next;
             const T b_p2 = pf_b;
@@ -198,7 +184,7 @@ __global__ void __launch_bounds__(256, MINB) dense_march_kernel(DenseK<T> p) {
             }
 
             if (out_lane) {
-                const bool inside = LEAN || (p.mask == nullptr) || (p.mask[(int64_t)r * p.mpitch + c] != 0);
+                const bool inside = (p.mask == nullptr) || (p.mask[(int64_t)r * p.mpitch + c] != 0);
                 if (!inside) { rh = (T)0; rhu = (T)0; rhv = (T)0; }
                 const int64_t o = (int64_t)r * p.pitch + c;
                 if (!STEP) {
@@ -207,32 +193,26 @@ __global__ void __launch_bounds__(256, MINB) dense_march_kernel(DenseK<T> p) {
                     T rr0 = rh;
                     if (inside) {
                         if (p.rain_kind == GSW_RAIN_UNIFORM) rr0 = rh + rate;
-                        else if (!LEAN && p.rain_kind == GSW_RAIN_GRIDDED)
+                        else if (p.rain_kind == GSW_RAIN_GRIDDED)
                             rr0 = rh + frame[(int64_t)(r - p.ngh) * (p.nyp - 2 * p.ngh) + (c - p.ngh)];
                     }
                     T h = cur.h + dt * rr0;
                     T hu = ldg_at(p.q1, p.pitch, r, c) + dt * rhu;     // reloaded: not carried down the march
                     T hv = ldg_at(p.q2, p.pitch, r, c) + dt * rhv;
                     T n = (T)0;
-                    if (LEAN) n = p.ntab[cls_r];
-                    else if (p.friction_kind == GSW_FRICTION_TABLE)
+                    if (p.friction_kind == GSW_FRICTION_TABLE)
                         n = p.ncls ? p.ntab[p.ncls[(int64_t)r * p.cpitch + c]] : p.ntab[0];
                     else if (p.friction_kind == GSW_FRICTION_FIELD) n = p.nfield[o];
-                    wetdry_friction<T>(h, hu, hv, LEAN || p.friction_kind != GSW_FRICTION_NONE, n, dt, p.g,
-                                       p.h_min, p.vcap, LEAN || p.quad != 0, LEAN || p.keep_h != 0, REFPOW);
+                    wetdry_friction<T>(h, hu, hv, p.friction_kind != GSW_FRICTION_NONE, n, dt, p.g,
+                                       p.h_min, p.vcap, p.quad != 0, p.keep_h != 0, REFPOW);
                     p.o0[o] = h; p.o1[o] = hu; p.o2[o] = hv;
-                    if (LEAN) { if (p.max_h != nullptr && h > mh_r) p.max_h[o] = h; }
-                    else if (p.max_h != nullptr && h > p.max_h[o]) p.max_h[o] = h;
-                    if (LEAN || p.lam != nullptr) {
-                        const bool skip = !LEAN && (p.cfl_skip != nullptr) &&
+                    if (p.max_h != nullptr && h > p.max_h[o]) p.max_h[o] = h;
+                    if (p.lam != nullptr) {
+                        const bool skip = (p.cfl_skip != nullptr) &&
                             p.cfl_skip[(int64_t)(r - p.ngh) * (p.nyp - 2 * p.ngh) + (c - p.ngh)] != 0;
                         if (!skip) {
-                            if constexpr (sizeof(T) == 4) {
-                                lam32 = max(lam32, lam_dense_bits32(h, hu, hv, p.g, p.h_cfl));
-                            } else {
-                                const unsigned long long lb = lam_dense_bits(h, hu, hv, p.g, p.h_cfl);
-                                lam_local = lb > lam_local ? lb : lam_local;
-                            }
+                            const unsigned long long lb = lam_dense_bits(h, hu, hv, p.g, p.h_cfl);
+                            lam_local = lb > lam_local ? lb : lam_local;
                         }
                     }
                 }
@@ -241,8 +221,118 @@ __global__ void __launch_bounds__(256, MINB) dense_march_kernel(DenseK<T> p) {
             b_next = b_p2;
         }
     }
-    if constexpr (sizeof(T) == 4) lam_local = lam_bits_of32(lam32);
-    if (STEP && (LEAN || p.lam != nullptr)) block_max_to(lam_local, p.lam);
+    if (STEP && p.lam != nullptr) block_max_to(lam_local, p.lam);
+}
+
+// ------------------------------------------------------------------- binary32 (march_rows)
+// The rows of one warp's tile. The plane pointers are taken at the tile's first row (uniform
+// over the block), so a lane's offsets are 32-bit.
+struct DenseRows {
+    const float* q0; const float* q1; const float* q2; const float* b;
+    int pitch, cl, co;           // cl: the lane's column, co: the one beyond the halo column
+    __device__ __forceinline__ void state(int k, float& h, float& hu, float& hv) const {
+        const int o = k * pitch + cl;
+        h = __ldg(q0 + o); hu = __ldg(q1 + o); hv = __ldg(q2 + o);
+    }
+    __device__ __forceinline__ float bed(int k) const { return __ldg(b + (k * pitch + cl)); }
+    __device__ __forceinline__ float bed_out(int k) const { return __ldg(b + (k * pitch + co)); }
+};
+
+// A row's update (STEP) or its residual. REFPOW: Manning's h^(-4/3) by powf (GSW_ARITH_EXACT)
+// instead of pow_m43. LEAN: the production configuration (no inside mask, no CFL skip mask,
+// the wave speed reduced, a Manning class table, quadratic friction, keep-h; rain none or
+// uniform), with those choices compiled in rather than tested per cell. Any other
+// configuration takes the general kernel; both give the same bits.
+template <bool STEP, bool REFPOW, bool LEAN>
+struct DenseRow {
+    const DenseK<float>& p;
+    int c, i0;
+    bool out_lane;
+    float dt, rate;
+    const float* frame;
+    uint32_t lam = 0u;           // the bits of the largest wave speed
+    uint8_t cls = 0;
+    float mh = 0.0f;
+
+    __device__ __forceinline__ float manning(int64_t r, int64_t o) const {
+        if (p.friction_kind == GSW_FRICTION_TABLE) return p.ncls ? p.ntab[p.ncls[r * p.cpitch + c]] : p.ntab[0];
+        return p.friction_kind == GSW_FRICTION_FIELD ? p.nfield[o] : 0.0f;
+    }
+    __device__ __forceinline__ int64_t interior(int64_t r) const {
+        return (r - p.ngh) * (int64_t)(p.nyp - 2 * p.ngh) + (c - p.ngh);
+    }
+    __device__ __forceinline__ void pre(int k) {
+        // the update's class id and running maximum, loaded before the faces so that their
+        // latency is hidden (the production kernel; the general one loads late)
+        if (LEAN && STEP && out_lane) {
+            cls = (p.ncls + (int64_t)i0 * p.cpitch)[k * (int)p.cpitch + c];
+            if (p.max_h != nullptr) mh = (p.max_h + (int64_t)i0 * p.pitch)[k * (int)p.pitch + c];
+        }
+    }
+    __device__ __forceinline__ void row(int k, float h, float rh, float rhu, float rhv) {
+        if (!out_lane) return;
+        const int64_t base = (int64_t)i0 * p.pitch, r = i0 + k;
+        const int o = k * (int)p.pitch + c;
+        const bool inside = LEAN || p.mask == nullptr || p.mask[r * p.mpitch + c] != 0;
+        if (!inside) { rh = 0.0f; rhu = 0.0f; rhv = 0.0f; }
+        if (!STEP) {
+            (p.o0 + base)[o] = rh; (p.o1 + base)[o] = rhu; (p.o2 + base)[o] = rhv;
+            return;
+        }
+        if (inside) {
+            if (p.rain_kind == GSW_RAIN_UNIFORM) rh = rh + rate;
+            else if (!LEAN && p.rain_kind == GSW_RAIN_GRIDDED) rh = rh + frame[interior(r)];
+        }
+        FState s;
+        s.h = h + dt * rh;
+        s.hu = __ldg(p.q1 + base + o) + dt * rhu;     // reloaded: not carried down the march
+        s.hv = __ldg(p.q2 + base + o) + dt * rhv;
+        const float n = LEAN ? p.ntab[cls] : manning(r, r * p.pitch + c);
+        const bool fric = LEAN || p.friction_kind != GSW_FRICTION_NONE;
+        bool slow = p.general || (!LEAN && (p.quad == 0 || p.keep_h == 0));
+        if (!slow) slow = update_in<false, REFPOW>(s, fric, n, dt, p.g, p.h_min, p.vcap, p.h_cfl);
+        if (slow) {
+            FState g = s;                               // a copy: s itself stays in registers
+            update_general<false, REFPOW>(g, fric, n, dt, p.g, p.h_min, p.vcap, LEAN || p.quad != 0,
+                                          LEAN || p.keep_h != 0, p.h_cfl);
+            s = g;
+        }
+        (p.o0 + base)[o] = s.h; (p.o1 + base)[o] = s.hu; (p.o2 + base)[o] = s.hv;
+        if (p.max_h != nullptr) {
+            float& m = (p.max_h + base)[o];
+            if (s.h > (LEAN ? mh : m)) m = s.h;
+        }
+        if (LEAN || p.cfl_skip == nullptr || p.cfl_skip[interior(r)] == 0) lam = max(lam, s.lam);
+    }
+};
+
+template <bool STEP, int REGS, bool REFPOW, bool LEAN>
+__global__ void __maxnreg__(REGS) dense_rows_kernel(DenseK<float> p) {
+    if (STEP && p.st->done) return;                       // grid-uniform
+    const int lane = threadIdx.x;
+    const int strip = blockIdx.x * blockDim.y + threadIdx.y;
+    const int col0 = p.col_lo + strip * 30;
+    const bool warp_active = col0 < p.col_hi;
+    const int c = col0 - 1 + lane;
+    const int i0 = p.row_lo + blockIdx.y * p.tile_rows;
+    const int n = min(p.tile_rows, p.row_hi - i0);
+    DenseRow<STEP, REFPOW, LEAN> upd = {p, c, i0, warp_active && lane >= 1 && lane <= 30 && c < p.col_hi,
+                                        0.0f, 0.0f, nullptr};
+    if (STEP) {
+        upd.dt = p.st->dt_f32;
+        if (p.rain_kind == GSW_RAIN_UNIFORM) upd.rate = p.rain[p.st->rain_idx];
+        if (p.rain_kind == GSW_RAIN_GRIDDED)
+            upd.frame = p.rain + (int64_t)p.st->rain_idx * (int64_t)(p.nxp - 2 * p.ngh) * (p.nyp - 2 * p.ngh);
+    }
+    if (warp_active && n > 0) {
+        const int64_t base = (int64_t)i0 * p.pitch;
+        const DenseRows acc = {p.q0 + base, p.q1 + base, p.q2 + base, p.b + base, (int)p.pitch, min(c, p.nyp - 1),
+                               lane == 0 ? max(c - 1, 0) : min(c + 1, p.nyp - 1)};
+        const FacePhys ph = {p.inv_dx, p.inv_dy, 0.5f * p.inv_dx, 0.5f * p.inv_dy, p.half_dx, p.half_dy,
+                             p.g, p.g_recip != 0.0f ? p.g_recip : rcp_in(p.g), p.h_min};
+        march_rows(acc, upd, n, ph, p.general);
+    }
+    if (STEP && (LEAN || p.lam != nullptr)) warp_max_to(lam_bits_of32(upd.lam), p.lam);
 }
 
 template <typename T>
@@ -285,6 +375,7 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
     k.ntab = (const T*)a->n_tab; k.nfield = (const T*)a->n_field;
     k.vcap = (T)a->vcap; k.quad = a->quadratic; k.keep_h = a->keep_h;
     k.max_h = (T*)a->max_h; k.cfl_skip = a->cfl_skip; k.h_cfl = (T)a->h_cfl;
+    k.general = !face_ranges((float)k.g, (float)k.h_min, (float)k.h_cfl);
     if (a->tile_rows > 0) {
         k.tile_rows = a->tile_rows;
     } else {   // rows per warp: the longest march (<= 32 rows) that still gives twice the resident warps
@@ -294,6 +385,10 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
         for (int tr = 32; tr > 4; tr >>= 1)
             if (strips * ((nrows + tr - 1) / tr) >= want) { k.tile_rows = tr; break; }
     }
+    // dense_rows_kernel's offsets within a tile (rows -2 .. tile_rows + 1) are 32-bit
+    const int64_t widest = std::max(k.pitch, std::max(k.cpitch, (int64_t)1));
+    k.long_rows = INT32_MAX / widest < 5;
+    if (!k.long_rows) k.tile_rows = (int)std::min<int64_t>(k.tile_rows, INT32_MAX / widest - 4);
     if (step) {
         if (!a->state) return set_error(GSW_ERR_INVALID, "dense step: state (GswLoopState*) is required");
         if (a->rain_kind != GSW_RAIN_NONE && a->rain_kind != GSW_RAIN_UNIFORM && a->rain_kind != GSW_RAIN_GRIDDED)
@@ -309,28 +404,30 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
     return GSW_OK;
 }
 
-template <typename T, bool STEP, bool REFPOW, bool LEAN>
-inline void launch_march_caps(const DenseK<T>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
-    // register caps apply to the binary32 step; the residual and binary64 use the compiler's choice
-    constexpr bool capped = STEP && sizeof(T) == 4;
-    if (capped && minb == 3) dense_march_kernel<T, STEP, capped ? 3 : 1, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
-    else if (capped && minb == 4) dense_march_kernel<T, STEP, capped ? 4 : 1, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
-    else if (capped && minb == 5) dense_march_kernel<T, STEP, capped ? 5 : 1, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
-    else dense_march_kernel<T, STEP, 1, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
-}
-
 // The production configuration (the LEAN kernel) or the general kernel.
-template <typename T>
-inline bool lean_config(const DenseK<T>& k) {
+inline bool lean_config(const DenseK<float>& k) {
     return k.mask == nullptr && k.cfl_skip == nullptr && k.lam != nullptr && k.friction_kind == GSW_FRICTION_TABLE &&
            k.ncls != nullptr && k.rain_kind != GSW_RAIN_GRIDDED && k.quad != 0 && k.keep_h != 0;
 }
 
-template <typename T, bool STEP, bool REFPOW>
-inline void launch_march_shape(const DenseK<T>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
-    constexpr bool can_lean = STEP && sizeof(T) == 4;
-    if (can_lean && lean_config(k)) launch_march_caps<T, STEP, REFPOW, can_lean>(k, minb, grid, block, s);
-    else launch_march_caps<T, STEP, REFPOW, false>(k, minb, grid, block, s);
+// Register caps of the binary32 step by GswDenseArgs.min_blocks.
+template <bool STEP, bool REFPOW, bool LEAN>
+inline void launch_rows_caps(const DenseK<float>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
+    if (STEP && minb == 3) dense_rows_kernel<STEP, STEP ? 96 : 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
+    else if (STEP && minb == 4) dense_rows_kernel<STEP, STEP ? 64 : 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
+    else if (STEP && minb == 5) dense_rows_kernel<STEP, STEP ? 72 : 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
+    else dense_rows_kernel<STEP, 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
+}
+
+template <bool STEP, bool REFPOW>
+inline void launch_shape(const DenseK<float>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
+    if (k.long_rows) dense_march_kernel<float, STEP, REFPOW><<<grid, block, 0, s>>>(k);
+    else if (STEP && lean_config(k)) launch_rows_caps<STEP, REFPOW, STEP>(k, minb, grid, block, s);
+    else launch_rows_caps<STEP, REFPOW, false>(k, minb, grid, block, s);
+}
+template <bool STEP, bool REFPOW>
+inline void launch_shape(const DenseK<double>& k, int, dim3 grid, dim3 block, cudaStream_t s) {
+    dense_march_kernel<double, STEP, false><<<grid, block, 0, s>>>(k);
 }
 
 template <typename T, bool STEP>
@@ -348,8 +445,8 @@ inline int launch_march(const GswDenseArgs* a, cudaStream_t s) {
     dim3 grid((strips + W - 1) / W, (nrows + k.tile_rows - 1) / k.tile_rows);
     if (grid.y > 65535u) return set_error(GSW_ERR_INVALID, "dense: too many row tiles (%u); raise tile_rows", grid.y);
     constexpr bool can_refpow = kRefPowBuild && STEP && sizeof(T) == 4;
-    if (can_refpow && a->arith == GSW_ARITH_EXACT) launch_march_shape<T, STEP, can_refpow>(k, minb, grid, block, s);
-    else launch_march_shape<T, STEP, false>(k, minb, grid, block, s);
+    if (can_refpow && a->arith == GSW_ARITH_EXACT) launch_shape<STEP, can_refpow>(k, minb, grid, block, s);
+    else launch_shape<STEP, false>(k, minb, grid, block, s);
     return check_launch("dense_march");
 }
 

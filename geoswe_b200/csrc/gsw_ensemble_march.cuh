@@ -75,8 +75,8 @@ __device__ __forceinline__ void build_run_list(const GswEnsembleArgs& a, int tid
 
 // LEAN: every member in the production configuration (quadratic friction, keep-h, the L2
 // norm; members take rain none or uniform), compiled in as in the stand-alone flat step.
-template <int MINB, bool REFPOW, bool LEAN>
-__global__ void __launch_bounds__(256, MINB) ensemble_step_kernel(GswEnsembleArgs a, FlatMesh<float> m) {
+template <typename I, int REGS, bool REFPOW, bool LEAN>
+__global__ void __maxnreg__(REGS) ensemble_step_kernel(GswEnsembleArgs a, FlatMesh<float> m) {
     if (*a.all_done) return;
     const int lane = threadIdx.x;
     const int W = blockDim.y;
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(256, MINB) ensemble_step_kernel(GswEnsembleArg
         const FlatPhys<float> ph = member_phys(mb, REFPOW ? 1 : 0);
         const float dt = st->dt_f32;
         const float rate = (mb.rain_kind == GSW_RAIN_UNIFORM) ? mb.rain[st->rain_idx] : 0.0f;
-        unsigned long long lam = flat_brick<float, true, REFPOW, LEAN>(m, ph, b, seg * m.bh / S, (seg + 1) * m.bh / S,
-                                                               dt, rate, nullptr);
+        unsigned long long lam = flat_brick<float, I, true, REFPOW, LEAN>(m, ph, b, seg * m.bh / S, (seg + 1) * m.bh / S,
+                                                                  dt, rate, nullptr);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long w = __shfl_xor_sync(0xffffffffu, lam, o);
@@ -165,12 +165,16 @@ __global__ void __launch_bounds__(256, MINB) ensemble_step_kernel(GswEnsembleArg
     }
 }
 
+// Register caps by GswEnsembleArgs.min_blocks; 64-bit slots where the storage needs them.
 template <bool REFPOW, bool LEAN>
 inline void launch_ensemble_caps(const GswEnsembleArgs* a, const FlatMesh<float>& m, int grid, int W, cudaStream_t st) {
-    if (a->min_blocks == 3) ensemble_step_kernel<3, REFPOW, LEAN><<<grid, dim3(32, W), 0, st>>>(*a, m);
-    else if (a->min_blocks == 4) ensemble_step_kernel<4, REFPOW, LEAN><<<grid, dim3(32, W), 0, st>>>(*a, m);
-    else if (a->min_blocks == 5) ensemble_step_kernel<5, REFPOW, LEAN><<<grid, dim3(32, W), 0, st>>>(*a, m);
-    else ensemble_step_kernel<1, REFPOW, LEAN><<<grid, dim3(32, W), 0, st>>>(*a, m);
+    const dim3 b(32, W);
+    if ((m.nb + 1) * (int64_t)m.bh * GSW_BRICK_PITCH > INT32_MAX)
+        ensemble_step_kernel<int64_t, 128, REFPOW, LEAN><<<grid, b, 0, st>>>(*a, m);
+    else if (a->min_blocks == 3) ensemble_step_kernel<int, 80, REFPOW, LEAN><<<grid, b, 0, st>>>(*a, m);
+    else if (a->min_blocks == 4) ensemble_step_kernel<int, 64, REFPOW, LEAN><<<grid, b, 0, st>>>(*a, m);
+    else if (a->min_blocks == 5) ensemble_step_kernel<int, 72, REFPOW, LEAN><<<grid, b, 0, st>>>(*a, m);
+    else ensemble_step_kernel<int, 96, REFPOW, LEAN><<<grid, b, 0, st>>>(*a, m);
 }
 
 template <bool REFPOW>

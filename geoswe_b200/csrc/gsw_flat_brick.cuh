@@ -2,6 +2,7 @@
 // solver's kernels and the ensemble's persistent step).
 #pragma once
 #include "gsw_common.cuh"
+#include "gsw_face.cuh"
 
 namespace gsw {
 
@@ -107,29 +108,124 @@ __device__ __forceinline__ Face<T> shfl_up_face(const Face<T>& f) {
     return r;
 }
 
-// Rows [r0, r1) of one brick, walked by one warp (T = float; double serves the adjoint's
-// fp64 checks). A segment reads rows r0-2 .. r1+1 through the brick view (the bricks
-// above and below past the brick's edge) and recomputes the x-face above row r0 from
-// the same inputs as the face below row r0-1, so splitting a brick's rows among warps
-// changes no value. STEP: the fused step (returns this lane's wave speed bits);
-// otherwise the residual. `frame` is the gridded rain frame, or null. REFPOW: Manning's
-// h^(-4/3) by powf (GSW_ARITH_EXACT) instead of pow_m43. LEAN: the production
-// configuration compiled in (rain none or uniform, quadratic friction, keep-h, the L2
-// wave-speed norm); the same bits as the general path.
-template <typename T, bool STEP, bool REFPOW, bool LEAN = false>
-__device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, const FlatPhys<T>& ph, int64_t bidx,
-                                                         int r0, int r1, T dt, T rate, const T* frame) {
+// Slots of one lane's rows of a brick, as BrickView::slot, by one base per row range. I: the
+// slots' integer type, 32-bit where the mesh has fewer than 2^31 slots (a 64-bit base costs
+// registers and address arithmetic on every access), else 64-bit.
+template <typename I>
+struct FlatRows {
+    const FlatMesh<float>& m;
+    I in, up, down, out;             // slots of row 0 continued from inside / above / below; lane 0/31: beyond
+    I zero;
+    int r0, bh;
+    __device__ __forceinline__ I slot(int r) const {
+        return (r < 0 ? up : (r >= bh ? down : in)) + (I)(r * GSW_BRICK_PITCH);
+    }
+    __device__ __forceinline__ void state(int k, float& h, float& hu, float& hv) const {
+        const I s = slot(r0 + k);
+        h = __ldg(m.q0 + s); hu = __ldg(m.q1 + s); hv = __ldg(m.q2 + s);
+    }
+    __device__ __forceinline__ float bed(int k) const { return __ldg(m.b + slot(r0 + k)); }
+    __device__ __forceinline__ float bed_out(int k) const {
+        const int r = r0 + k;
+        return __ldg(m.b + (r < 0 || r >= bh ? zero : out + (I)(r * GSW_BRICK_PITCH)));
+    }
+};
+
+template <typename I>
+__device__ __forceinline__ FlatRows<I> flat_rows(const FlatMesh<float>& m, const BrickView& v, int r0, int lane) {
+    const I BS = (I)(v.bh * GSW_BRICK_PITCH);
+    FlatRows<I> a = {m, 0, 0, 0, 0, (I)v.zero * BS, r0, v.bh};
+    const bool halo = lane == 0 || lane == 31;
+    a.in = lane == 0 ? (I)v.left * BS + (GSW_BRICK_W - 1) : lane == 31 ? (I)v.right * BS : (I)v.self * BS + (lane - 1);
+    a.up = (halo ? a.zero : (I)v.up * BS + (lane - 1)) + BS;         // halo lanes read the zero brick there
+    a.down = (halo ? a.zero : (I)v.down * BS + (lane - 1)) - BS;
+    a.out = lane == 0 ? (I)v.left * BS + (GSW_BRICK_W - 2) : (I)v.right * BS + 1;
+    return a;
+}
+
+// One row's update (STEP) or its residual. REFPOW: Manning's h^(-4/3) by powf
+// (GSW_ARITH_EXACT) instead of pow_m43. LEAN: the production configuration compiled in (rain
+// none or uniform, quadratic friction, keep-h, the L2 wave-speed norm); the same bits as the
+// general path.
+template <typename I, bool STEP, bool REFPOW, bool LEAN>
+struct FlatRow {
+    const FlatMesh<float>& m;
+    const FlatPhys<float>& ph;
+    I base;                          // the lane's slot of row 0
+    int bi, bj, r0, lane;
+    float dt, rate;
+    const float* frame;
+    bool general;
+    bool out_lane;
+    uint32_t lam32 = 0u;             // the L2 norm's key
+    unsigned long long lam64 = 0ull; // the general kernel's (either norm)
+    uint8_t f = 0, cls = 0;
+    float mh = 0.0f;
+    __device__ __forceinline__ void pre(int k) {
+        // the slot flag, class id and running maximum, loaded before the faces so that their
+        // latency is hidden (the production kernel; the general one loads late)
+        if (LEAN && STEP && out_lane) {
+            const I o = base + (I)((r0 + k) * GSW_BRICK_PITCH);
+            f = m.flags[o];
+            if (m.ncls) cls = m.ncls[o];
+            if (m.max_h != nullptr) mh = m.max_h[o];
+        }
+    }
+    __device__ __forceinline__ void row(int k, float h, float rh, float rhu, float rhv) {
+        if (!out_lane) return;
+        const I o = base + (I)((r0 + k) * GSW_BRICK_PITCH);
+        const uint8_t fl = (LEAN && STEP) ? f : m.flags[o];
+        if (!(fl & GSW_SLOT_STORED)) return;
+        const bool active = (fl & GSW_SLOT_ACTIVE) != 0;
+        if (!STEP) {
+            m.o0[o] = active ? rh : 0.0f; m.o1[o] = active ? rhu : 0.0f; m.o2[o] = active ? rhv : 0.0f;
+            return;
+        }
+        FState s;
+        s.h = h;
+        s.hu = __ldg(m.q1 + o);                       // reloaded: not carried down the march
+        s.hv = __ldg(m.q2 + o);
+        if (active) {
+            if (ph.rain_kind == GSW_RAIN_UNIFORM) rh = rh + rate;
+            else if (!LEAN && ph.rain_kind == GSW_RAIN_GRIDDED) {
+                const int i = bi * m.bh + r0 + k, j = bj * GSW_BRICK_W + (lane - 1);
+                rh = rh + frame[(int64_t)(i - ph.ngh) * ph.ny + (j - ph.ngh)];
+            } else if (!LEAN && ph.rain_kind == GSW_RAIN_LOOKUP) {
+                rh = rh + frame[ph.lookup[o]];
+            }
+            s.h = h + dt * rh;
+            s.hu = s.hu + dt * rhu;
+            s.hv = s.hv + dt * rhv;
+            const float n = m.ncls ? ph.ntab[LEAN ? cls : m.ncls[o]] : ph.ntab[0];
+            bool slow = general || (!LEAN && (ph.quad == 0 || ph.keep_h == 0));
+            if (!slow) slow = update_in<true, REFPOW>(s, true, n, dt, ph.g, ph.h_min, ph.vcap, ph.h_min);
+            if (slow) {
+                FState g = s;                         // a copy: s itself stays in registers
+                update_general<true, REFPOW>(g, true, n, dt, ph.g, ph.h_min, ph.vcap, LEAN || ph.quad != 0,
+                                             LEAN || ph.keep_h != 0, ph.h_min_cfl);
+                s = g;
+            }
+            if (LEAN || ph.linf == 0) {
+                lam32 = max(lam32, s.lam);
+            } else {
+                const unsigned long long lb = lam_flat_bits(s.h, s.hu, s.hv, ph.g, ph.h_min, ph.h_min_cfl, true);
+                lam64 = lb > lam64 ? lb : lam64;
+            }
+        }
+        m.o0[o] = s.h; m.o1[o] = s.hu; m.o2[o] = s.hv;
+        if (m.max_h != nullptr && s.h > (LEAN ? mh : m.max_h[o])) m.max_h[o] = s.h;
+    }
+};
+
+// Rows [r0, r1) of one brick in binary64 (the adjoint's derivative checks).
+template <bool STEP>
+__device__ __forceinline__ unsigned long long flat_brick_f64(const FlatMesh<double>& m, const FlatPhys<double>& ph,
+                                                             const BrickView& v, int bi, int bj, int r0, int r1,
+                                                             double dt, double rate, const double* frame) {
+    using T = double;
     const int lane = threadIdx.x;
+    const int64_t bidx = v.self;
     unsigned long long lam_local = 0ull;
-    uint32_t lam32 = 0u;        // the production kernel's binary32 key (lam_flat_bits32)
-    BrickView v;
-    v.BS = (int64_t)m.bh * GSW_BRICK_PITCH;
-    v.bh = m.bh;
-    v.self = bidx;
-    v.up = m.bnbr[4 * bidx + 0]; v.down = m.bnbr[4 * bidx + 1];
-    v.left = m.bnbr[4 * bidx + 2]; v.right = m.bnbr[4 * bidx + 3];
-    v.zero = m.nb;
-    const int bi = m.bij[2 * bidx], bj = m.bij[2 * bidx + 1];
     const int bh = m.bh;
     Cell<T> cur, nx;
     const T b_m2 = __ldg(m.b + v.slot(r0 - 2, lane));
@@ -150,16 +246,6 @@ __device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, c
     srm_face<T, true>(cur, nx, ph.half_dx, ph.inv_dx, ph.g, ph.h_min, Wf, ph.g_recip);
     cur = nx;
     for (int r = r0; r < r1; ++r) {
-        // the update's slot flag, class id and running maximum, loaded before the faces so
-        // that their latency is hidden (the production kernel; the general one loads late)
-        uint8_t f_r = 0, cls_r = 0;
-        T mh_r = (T)0;
-        if (LEAN && STEP && lane >= 1 && lane <= 30) {
-            const int64_t o = bidx * v.BS + (int64_t)r * GSW_BRICK_PITCH + (lane - 1);
-            f_r = m.flags[o];
-            if (m.ncls) cls_r = m.ncls[o];
-            if (m.max_h != nullptr) mh_r = m.max_h[o];
-        }
         nx.h = pf_h; nx.hu = pf_hu; nx.hv = pf_hv;
         nx.b = b_next;
         const T b_p2 = pf_b;
@@ -194,7 +280,7 @@ __device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, c
         }
         if (lane >= 1 && lane <= 30) {
             const int64_t o = bidx * v.BS + (int64_t)r * GSW_BRICK_PITCH + (lane - 1);
-            const uint8_t f = (LEAN && STEP) ? f_r : m.flags[o];
+            const uint8_t f = m.flags[o];
             if (f & GSW_SLOT_STORED) {
                 const bool active = (f & GSW_SLOT_ACTIVE) != 0;
                 if (!STEP) {
@@ -202,39 +288,65 @@ __device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, c
                     m.o0[o] = rh; m.o1[o] = rhu; m.o2[o] = rhv;
                 } else if (!active) {
                     m.o0[o] = cur.h; m.o1[o] = __ldg(m.q1 + o); m.o2[o] = __ldg(m.q2 + o);
-                    if (m.max_h != nullptr && cur.h > (LEAN ? mh_r : m.max_h[o])) m.max_h[o] = cur.h;
+                    if (m.max_h != nullptr && cur.h > m.max_h[o]) m.max_h[o] = cur.h;
                 } else {
                     T rr0 = rh;
                     if (ph.rain_kind == GSW_RAIN_UNIFORM) rr0 = rr0 + rate;
-                    else if (!LEAN && ph.rain_kind == GSW_RAIN_GRIDDED) {
+                    else if (ph.rain_kind == GSW_RAIN_GRIDDED) {
                         const int i = bi * bh + r, j = bj * GSW_BRICK_W + (lane - 1);
                         rr0 = rr0 + frame[(int64_t)(i - ph.ngh) * ph.ny + (j - ph.ngh)];
-                    } else if (!LEAN && ph.rain_kind == GSW_RAIN_LOOKUP) {
+                    } else if (ph.rain_kind == GSW_RAIN_LOOKUP) {
                         rr0 = rr0 + frame[ph.lookup[o]];
                     }
                     T h = cur.h + dt * rr0;
                     T hu = __ldg(m.q1 + o) + dt * rhu;       // reloaded: not carried down the march
                     T hv = __ldg(m.q2 + o) + dt * rhv;
-                    const T n = m.ncls ? ph.ntab[LEAN ? cls_r : m.ncls[o]] : ph.ntab[0];
+                    const T n = m.ncls ? ph.ntab[m.ncls[o]] : ph.ntab[0];
                     wetdry_friction<T>(h, hu, hv, true, n, dt, ph.g, ph.h_min, ph.vcap,
-                                       LEAN || ph.quad != 0, LEAN || ph.keep_h != 0, REFPOW);
+                                       ph.quad != 0, ph.keep_h != 0, false);
                     m.o0[o] = h; m.o1[o] = hu; m.o2[o] = hv;
-                    if (m.max_h != nullptr && h > (LEAN ? mh_r : m.max_h[o])) m.max_h[o] = h;
-                    if constexpr (LEAN && sizeof(T) == 4) {
-                        lam32 = max(lam32, lam_flat_bits32(h, hu, hv, ph.g, ph.h_min, ph.h_min_cfl));
-                    } else {
-                        const unsigned long long lb = lam_flat_bits(h, hu, hv, ph.g, ph.h_min, ph.h_min_cfl,
-                                                                    !LEAN && ph.linf != 0);
-                        lam_local = lb > lam_local ? lb : lam_local;
-                    }
+                    if (m.max_h != nullptr && h > m.max_h[o]) m.max_h[o] = h;
+                    const unsigned long long lb = lam_flat_bits(h, hu, hv, ph.g, ph.h_min, ph.h_min_cfl, ph.linf != 0);
+                    lam_local = lb > lam_local ? lb : lam_local;
                 }
             }
         }
         cur = nx;
         b_next = b_p2;
     }
-    if constexpr (LEAN && sizeof(T) == 4) lam_local = lam_bits_of32(lam32);
     return lam_local;
+}
+
+// Rows [r0, r1) of one brick, walked by one warp. A segment reads rows r0-2 .. r1+1 through
+// the brick view (the bricks above and below past the brick's edge) and recomputes the x-face
+// above row r0 from the same inputs as the face below row r0-1, so splitting a brick's rows
+// among warps changes no value. STEP: the fused step (returns this lane's wave speed bits);
+// otherwise the residual. `frame` is the gridded rain frame, or null. I: as FlatRows.
+template <typename T, typename I, bool STEP, bool REFPOW, bool LEAN>
+__device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, const FlatPhys<T>& ph, int64_t bidx,
+                                                         int r0, int r1, T dt, T rate, const T* frame) {
+    const int lane = threadIdx.x;
+    BrickView v;
+    v.BS = (int64_t)m.bh * GSW_BRICK_PITCH;
+    v.bh = m.bh;
+    v.self = bidx;
+    v.up = m.bnbr[4 * bidx + 0]; v.down = m.bnbr[4 * bidx + 1];
+    v.left = m.bnbr[4 * bidx + 2]; v.right = m.bnbr[4 * bidx + 3];
+    v.zero = m.nb;
+    const int bi = m.bij[2 * bidx], bj = m.bij[2 * bidx + 1];
+    if constexpr (sizeof(T) == 4) {
+        const FlatRows<I> acc = flat_rows<I>(m, v, r0, lane);
+        const bool general = !face_ranges(ph.g, ph.h_min, ph.h_min_cfl) || ph.h_min_cfl != ph.h_min;
+        FlatRow<I, STEP, REFPOW, LEAN> upd = {m, ph, (I)(bidx * v.BS) + (lane - 1), bi, bj, r0, lane, dt, rate, frame, general,
+                                           lane >= 1 && lane <= 30};
+        const FacePhys fp = {ph.inv_dx, ph.inv_dy, 0.5f * ph.inv_dx, 0.5f * ph.inv_dy, ph.half_dx, ph.half_dy,
+                             ph.g, ph.g_recip != 0.0f ? ph.g_recip : rcp_in(ph.g), ph.h_min};
+        march_rows(acc, upd, r1 - r0, fp, general);
+        const unsigned long long l = lam_bits_of32(upd.lam32);
+        return LEAN || l > upd.lam64 ? l : upd.lam64;
+    } else {
+        return flat_brick_f64<STEP>(m, ph, v, bi, bj, r0, r1, dt, rate, frame);
+    }
 }
 
 }  // namespace gsw

@@ -14,8 +14,8 @@
 
 namespace gsw {
 
-template <typename T, bool STEP, int MINB, bool REFPOW, bool LEAN>
-__global__ void __launch_bounds__(256, MINB) flat_march_kernel(FlatK<T> p) {
+template <typename T, typename I, bool STEP, int REGS, bool REFPOW, bool LEAN>
+__global__ void __maxnreg__(REGS) flat_march_kernel(FlatK<T> p) {
     if (STEP && p.st->done) return;
     const int64_t item = (int64_t)blockIdx.x * blockDim.y + threadIdx.y;   // (brick, row segment)
     const int64_t rel = item / p.segs;
@@ -31,9 +31,9 @@ __global__ void __launch_bounds__(256, MINB) flat_march_kernel(FlatK<T> p) {
         if (p.ph.rain_kind == GSW_RAIN_LOOKUP) frame = p.ph.rain + (int64_t)p.st->rain_idx * p.ph.ncol;
     }
     if (bidx < p.b1)
-        lam_local = flat_brick<T, STEP, REFPOW, LEAN>(p.m, p.ph, bidx, seg * p.m.bh / p.segs, (seg + 1) * p.m.bh / p.segs,
-                                        dt, rate, frame);
-    if (STEP && p.lam != nullptr) block_max_to(lam_local, p.lam);
+        lam_local = flat_brick<T, I, STEP, REFPOW, LEAN>(p.m, p.ph, bidx, seg * p.m.bh / p.segs,
+                                                         (seg + 1) * p.m.bh / p.segs, dt, rate, frame);
+    if (STEP && p.lam != nullptr) warp_max_to(lam_local, p.lam);
 }
 
 template <typename T>
@@ -81,24 +81,30 @@ inline int fill_flat(const GswFlatArgs* a, FlatK<T>& k, bool step) {
     return GSW_OK;
 }
 
-template <typename T, bool STEP, bool REFPOW, bool LEAN>
-inline void launch_flat_caps(const FlatK<T>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
-    constexpr bool capped = STEP && sizeof(T) == 4;   // register caps apply to the binary32 step
-    if (capped && mb == 3) flat_march_kernel<T, STEP, capped ? 3 : 1, REFPOW, LEAN><<<blocks, dim3(32, W), 0, s>>>(k);
-    else if (capped && mb == 4) flat_march_kernel<T, STEP, capped ? 4 : 1, REFPOW, LEAN><<<blocks, dim3(32, W), 0, s>>>(k);
-    else if (capped && mb == 5) flat_march_kernel<T, STEP, capped ? 5 : 1, REFPOW, LEAN><<<blocks, dim3(32, W), 0, s>>>(k);
-    else flat_march_kernel<T, STEP, 1, REFPOW, LEAN><<<blocks, dim3(32, W), 0, s>>>(k);
+// Register caps of the binary32 step by GswFlatArgs.min_blocks.
+template <bool STEP, bool REFPOW, bool LEAN>
+inline void launch_flat_caps(const FlatK<float>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
+    const dim3 b(32, W);
+    if (STEP && mb == 3) flat_march_kernel<float, int, STEP, STEP ? 96 : 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
+    else if (STEP && mb == 4) flat_march_kernel<float, int, STEP, STEP ? 64 : 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
+    else if (STEP && mb == 5) flat_march_kernel<float, int, STEP, STEP ? 72 : 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
+    else flat_march_kernel<float, int, STEP, 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
 }
 
 // The production configuration (the LEAN kernel: rain none or uniform, quadratic
 // friction, keep-h, the L2 norm) or the general kernel.
-template <typename T, bool STEP, bool REFPOW>
-inline void launch_flat_shape(const FlatK<T>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
-    constexpr bool can_lean = STEP && sizeof(T) == 4;
+template <bool STEP, bool REFPOW>
+inline void launch_flat_shape(const FlatK<float>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
     const bool lean = k.ph.rain_kind != GSW_RAIN_GRIDDED && k.ph.rain_kind != GSW_RAIN_LOOKUP &&
                       k.ph.quad != 0 && k.ph.keep_h != 0 && k.ph.linf == 0;
-    if (can_lean && lean) launch_flat_caps<T, STEP, REFPOW, can_lean>(k, mb, blocks, W, s);
-    else launch_flat_caps<T, STEP, REFPOW, false>(k, mb, blocks, W, s);
+    if ((k.m.nb + 1) * (int64_t)k.m.bh * GSW_BRICK_PITCH > INT32_MAX)
+        flat_march_kernel<float, int64_t, STEP, 128, REFPOW, false><<<blocks, dim3(32, W), 0, s>>>(k);
+    else if (STEP && lean) launch_flat_caps<STEP, REFPOW, STEP>(k, mb, blocks, W, s);
+    else launch_flat_caps<STEP, REFPOW, false>(k, mb, blocks, W, s);
+}
+template <bool STEP, bool REFPOW>
+inline void launch_flat_shape(const FlatK<double>& k, int, unsigned blocks, int W, cudaStream_t s) {
+    flat_march_kernel<double, int64_t, STEP, 200, false, false><<<blocks, dim3(32, W), 0, s>>>(k);
 }
 
 template <typename T, bool STEP>
@@ -114,8 +120,8 @@ inline int launch_flat(const GswFlatArgs* a, cudaStream_t s) {
     const int mb = a->min_blocks;
     if (mb != 0 && (mb < 3 || mb > 5)) return set_error(GSW_ERR_INVALID, "flat: min_blocks must be 0, 3, 4 or 5");
     constexpr bool can_refpow = kRefPowBuild && STEP && sizeof(T) == 4;
-    if (can_refpow && a->arith == GSW_ARITH_EXACT) launch_flat_shape<T, STEP, can_refpow>(k, mb, (unsigned)blocks, W, s);
-    else launch_flat_shape<T, STEP, false>(k, mb, (unsigned)blocks, W, s);
+    if (can_refpow && a->arith == GSW_ARITH_EXACT) launch_flat_shape<STEP, can_refpow>(k, mb, (unsigned)blocks, W, s);
+    else launch_flat_shape<STEP, false>(k, mb, (unsigned)blocks, W, s);
     return check_launch("flat_march");
 }
 

@@ -172,8 +172,6 @@ class Solver2D:
             if best:
                 self._tile_rows, self._warps = int(best["tile_rows"]), int(best["warps"])
                 self._min_blocks = int(best["min_blocks"])
-            elif mesh.nx * mesh.ny >= 1 << 20:
-                self._min_blocks = 4     # untuned: the 64-register cap every large-grid tuning has chosen
         self._use_graphs = bool(use_graphs)
         dev, td = self.device, self.t_dtype
         self._buf = [torch.zeros((3, self.nxp, self.pitch), dtype=td, device=dev) for _ in range(2)]
