@@ -79,6 +79,7 @@ __device__ __forceinline__ void load_state(const FlatMesh<T>& m, int64_t s, Cell
 // ---------------------------------------------------------------------------- A
 template <typename T, int MINB>
 __global__ void __launch_bounds__(128, MINB) adj_tail_kernel(AdjK<T> p) {
+    chain_begin();
     __shared__ double s_nbar[256];
     __shared__ double s_rate[8];
     const int tid = threadIdx.x + 32 * threadIdx.y;
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(128, MINB) adj_tail_kernel(AdjK<T> p) {
 // ---------------------------------------------------------------------------- B
 template <typename T, int MINB>
 __global__ void __launch_bounds__(128, MINB) adj_face_kernel(AdjK<T> p) {
+    chain_begin();
     const FlatMesh<T>& m = p.m;
     const FlatPhys<T>& ph = p.ph;
     const int lane = threadIdx.x;
@@ -258,6 +260,7 @@ __global__ void __launch_bounds__(128, MINB) adj_face_kernel(AdjK<T> p) {
 // and to Q(t) of this step (q_bar[steps]); the ghost adjoints are then cleared.
 template <typename T>
 __global__ void adj_inflow_kernel(GswFlatInflowArgs a, T* l0, T* l1, T* l2, double* q_bar) {
+    chain_begin();
     if (threadIdx.x != 0) return;
     const T* q0 = (const T*)a.q0;
     const T* bed = (const T*)a.bed;
@@ -322,6 +325,7 @@ __global__ void adj_inflow_kernel(GswFlatInflowArgs a, T* l0, T* l1, T* l2, doub
 // ------------------------------------------------------------------------ gauges
 template <typename T>
 __global__ void gauge_record_kernel(GswGaugeArgs a) {
+    chain_begin();
     if (a.state != nullptr && a.state->done) return;
     const int64_t idx = (a.state ? a.state->steps : 0) + a.offset - a.first;
     if (idx < 0 || idx >= a.count) return;
@@ -333,6 +337,7 @@ __global__ void gauge_record_kernel(GswGaugeArgs a) {
 
 template <typename T>
 __global__ void gauge_adjoint_kernel(GswGaugeArgs a) {
+    chain_begin();
     const int64_t idx = (a.state ? a.state->steps : 0) + a.offset - a.first;
     if (idx < 0 || idx >= a.count) return;
     const T* q0 = (const T*)a.q0;
@@ -398,13 +403,13 @@ static int launch_adj(const GswFlatAdjArgs* a, cudaStream_t s) {
     const int mb = sizeof(T) == 4 ? a->min_blocks : 0;
     if (mb != 0 && mb != 6 && mb != 8) return set_error(GSW_ERR_INVALID, "adjoint: min_blocks must be 0, 6 or 8");
     const dim3 grid((unsigned)blocks), block(32, W);
-    if (mb == 6) adj_tail_kernel<T, sizeof(T) == 4 ? 6 : 1><<<grid, block, 0, s>>>(k);
-    else if (mb == 8) adj_tail_kernel<T, sizeof(T) == 4 ? 8 : 1><<<grid, block, 0, s>>>(k);
-    else adj_tail_kernel<T, 1><<<grid, block, 0, s>>>(k);
+    if (mb == 6) launch_chained(adj_tail_kernel<T, sizeof(T) == 4 ? 6 : 1>, grid, block, s, k);
+    else if (mb == 8) launch_chained(adj_tail_kernel<T, sizeof(T) == 4 ? 8 : 1>, grid, block, s, k);
+    else launch_chained(adj_tail_kernel<T, 1>, grid, block, s, k);
     if (int rc = check_launch("adj_tail")) return rc;
-    if (mb == 6) adj_face_kernel<T, sizeof(T) == 4 ? 6 : 1><<<grid, block, 0, s>>>(k);
-    else if (mb == 8) adj_face_kernel<T, sizeof(T) == 4 ? 8 : 1><<<grid, block, 0, s>>>(k);
-    else adj_face_kernel<T, 1><<<grid, block, 0, s>>>(k);
+    if (mb == 6) launch_chained(adj_face_kernel<T, sizeof(T) == 4 ? 6 : 1>, grid, block, s, k);
+    else if (mb == 8) launch_chained(adj_face_kernel<T, sizeof(T) == 4 ? 8 : 1>, grid, block, s, k);
+    else launch_chained(adj_face_kernel<T, 1>, grid, block, s, k);
     return check_launch("adj_face");
 }
 
@@ -425,9 +430,9 @@ extern "C" int gsw_adj_flat_inflow(const GswFlatInflowArgs* a, void* lam0, void*
         return set_error(GSW_ERR_INVALID, "adjoint inflow: null pointer, empty hydrograph or ds <= 0");
     cudaStream_t s = (cudaStream_t)stream;
     if (a->dtype == GSW_F32)
-        adj_inflow_kernel<float><<<1, 32, 0, s>>>(*a, (float*)lam0, (float*)lam1, (float*)lam2, q_bar);
+        launch_chained(adj_inflow_kernel<float>, dim3(1), dim3(32), s, *a, (float*)lam0, (float*)lam1, (float*)lam2, q_bar);
     else if (a->dtype == GSW_F64)
-        adj_inflow_kernel<double><<<1, 32, 0, s>>>(*a, (double*)lam0, (double*)lam1, (double*)lam2, q_bar);
+        launch_chained(adj_inflow_kernel<double>, dim3(1), dim3(32), s, *a, (double*)lam0, (double*)lam1, (double*)lam2, q_bar);
     else return set_error(GSW_ERR_INVALID, "adjoint inflow: bad dtype");
     return check_launch("adj_inflow");
 }
@@ -444,8 +449,8 @@ extern "C" int gsw_gauge_record(const GswGaugeArgs* a, void* stream) {
     if (!a->series) return set_error(GSW_ERR_INVALID, "gauge record: series is NULL");
     if (a->n == 0) return GSW_OK;
     const int grid = (a->n + 255) / 256;
-    if (a->dtype == GSW_F32) gauge_record_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(*a);
-    else gauge_record_kernel<double><<<grid, 256, 0, (cudaStream_t)stream>>>(*a);
+    if (a->dtype == GSW_F32) launch_chained(gauge_record_kernel<float>, dim3(grid), dim3(256), (cudaStream_t)stream, *a);
+    else launch_chained(gauge_record_kernel<double>, dim3(grid), dim3(256), (cudaStream_t)stream, *a);
     return check_launch("gauge_record");
 }
 
@@ -455,7 +460,7 @@ extern "C" int gsw_gauge_adjoint(const GswGaugeArgs* a, void* stream) {
     if (!a->target || !a->lam0) return set_error(GSW_ERR_INVALID, "gauge adjoint: target/lam0 is NULL");
     if (a->n == 0) return GSW_OK;
     const int grid = (a->n + 255) / 256;
-    if (a->dtype == GSW_F32) gauge_adjoint_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(*a);
-    else gauge_adjoint_kernel<double><<<grid, 256, 0, (cudaStream_t)stream>>>(*a);
+    if (a->dtype == GSW_F32) launch_chained(gauge_adjoint_kernel<float>, dim3(grid), dim3(256), (cudaStream_t)stream, *a);
+    else launch_chained(gauge_adjoint_kernel<double>, dim3(grid), dim3(256), (cudaStream_t)stream, *a);
     return check_launch("gauge_adjoint");
 }

@@ -5,6 +5,7 @@
 #include <stdarg.h>
 #include <stdio.h>
 #include <algorithm>
+#include <utility>
 #include "../../include/gsw.h"
 #include "gsw_core.cuh"
 
@@ -35,6 +36,13 @@ using gsw_rt::check_launch;
 using gsw_rt::sm_count;
 using gsw_rt::count_launch;
 using gsw_rt::div_const_recip;
+
+// Launch of a kernel of the time loop, and what each of them does first.
+__device__ __forceinline__ void chain_begin() {}
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
+    kernel<<<grid, block, 0, s>>>(std::forward<A>(args)...);
+}
 
 // Max of a non-negative IEEE-bits value over the block, then one atomicMax.
 // Every thread of the block must call it (it holds a block barrier).

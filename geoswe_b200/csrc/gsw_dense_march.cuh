@@ -101,6 +101,7 @@ template <> __device__ __forceinline__ double dt_of<double>(const GswLoopState* 
 // residual into o0..o2. STEP = true: updated state into o0..o2. REFPOW: as DenseRow's.
 template <typename T, bool STEP, bool REFPOW>
 __global__ void __launch_bounds__(256, 1) dense_march_kernel(DenseK<T> p) {
+    chain_begin();
     if (STEP && p.st->done) return;                       // grid-uniform
     const int lane = threadIdx.x;
     const int strip = blockIdx.x * blockDim.y + threadIdx.y;
@@ -308,6 +309,7 @@ struct DenseRow {
 
 template <bool STEP, int REGS, bool REFPOW, bool LEAN>
 __global__ void __maxnreg__(REGS) dense_rows_kernel(DenseK<float> p) {
+    chain_begin();
     if (STEP && p.st->done) return;                       // grid-uniform
     const int lane = threadIdx.x;
     const int strip = blockIdx.x * blockDim.y + threadIdx.y;
@@ -384,6 +386,11 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
         k.tile_rows = 4;
         for (int tr = 32; tr > 4; tr >>= 1)
             if (strips * ((nrows + tr - 1) / tr) >= want) { k.tile_rows = tr; break; }
+        // grids under four rows per resident warp: the shortest march that one wave of warps
+        // covers, since a step is then one march long (us per step, tile 4 against the rule's:
+        // 96^2 19.3 and 13.0 with one row, 256^2 19.3 and 14.8 with one, 512^2 24.5 and 23.7 with three)
+        if (sizeof(T) == 4 && strips * nrows < 4LL * sm_count() * 24)
+            k.tile_rows = (int)std::max<int64_t>(1, (strips * nrows + sm_count() * 24 - 1) / (sm_count() * 24));
     }
     // dense_rows_kernel's offsets within a tile (rows -2 .. tile_rows + 1) are 32-bit
     const int64_t widest = std::max(k.pitch, std::max(k.cpitch, (int64_t)1));
@@ -413,21 +420,21 @@ inline bool lean_config(const DenseK<float>& k) {
 // Register caps of the binary32 step by GswDenseArgs.min_blocks.
 template <bool STEP, bool REFPOW, bool LEAN>
 inline void launch_rows_caps(const DenseK<float>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
-    if (STEP && minb == 3) dense_rows_kernel<STEP, STEP ? 96 : 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
-    else if (STEP && minb == 4) dense_rows_kernel<STEP, STEP ? 64 : 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
-    else if (STEP && minb == 5) dense_rows_kernel<STEP, STEP ? 72 : 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
-    else dense_rows_kernel<STEP, 80, REFPOW, LEAN><<<grid, block, 0, s>>>(k);
+    if (STEP && minb == 3) launch_chained(dense_rows_kernel<STEP, STEP ? 96 : 80, REFPOW, LEAN>, grid, block, s, k);
+    else if (STEP && minb == 4) launch_chained(dense_rows_kernel<STEP, STEP ? 64 : 80, REFPOW, LEAN>, grid, block, s, k);
+    else if (STEP && minb == 5) launch_chained(dense_rows_kernel<STEP, STEP ? 72 : 80, REFPOW, LEAN>, grid, block, s, k);
+    else launch_chained(dense_rows_kernel<STEP, 80, REFPOW, LEAN>, grid, block, s, k);
 }
 
 template <bool STEP, bool REFPOW>
 inline void launch_shape(const DenseK<float>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
-    if (k.long_rows) dense_march_kernel<float, STEP, REFPOW><<<grid, block, 0, s>>>(k);
+    if (k.long_rows) launch_chained(dense_march_kernel<float, STEP, REFPOW>, grid, block, s, k);
     else if (STEP && lean_config(k)) launch_rows_caps<STEP, REFPOW, STEP>(k, minb, grid, block, s);
     else launch_rows_caps<STEP, REFPOW, false>(k, minb, grid, block, s);
 }
 template <bool STEP, bool REFPOW>
 inline void launch_shape(const DenseK<double>& k, int, dim3 grid, dim3 block, cudaStream_t s) {
-    dense_march_kernel<double, STEP, false><<<grid, block, 0, s>>>(k);
+    launch_chained(dense_march_kernel<double, STEP, false>, grid, block, s, k);
 }
 
 template <typename T, bool STEP>
@@ -435,7 +442,11 @@ inline int launch_march(const GswDenseArgs* a, cudaStream_t s) {
     DenseK<T> k;
     int rc = fill_dense<T>(a, k, STEP);
     if (rc) return rc;
-    const int W = a->warps > 0 ? a->warps : 4;
+    // two warps per block while the grid is under three waves of warps: the last wave then spreads
+    // over more SMs (fast arithmetic, us per step, 4 and 2 warps: 512^2 17.1 and 15.8, 1500^2 65.1
+    // and 63.2, 2500^2 141.6 and 143.1)
+    const int64_t tiles = (int64_t)((k.col_hi - k.col_lo + 29) / 30) * ((k.row_hi - k.row_lo + k.tile_rows - 1) / k.tile_rows);
+    const int W = a->warps > 0 ? a->warps : (sizeof(T) == 4 && tiles < 3LL * sm_count() * 24 ? 2 : 4);
     const int minb = a->min_blocks;
     if (minb != 0 && (minb < 3 || minb > 5)) return set_error(GSW_ERR_INVALID, "dense: min_blocks must be 0, 3, 4 or 5");
     if (W < 1 || W > 8) return set_error(GSW_ERR_INVALID, "dense: warps must be in [1, 8]");

@@ -8,6 +8,7 @@
 namespace gsw {
 
 __global__ void ensemble_finalize_kernel(GswEnsembleArgs a) {
+    chain_begin();
     __shared__ int s_open;
     if (threadIdx.x == 0) s_open = 0;
     __syncthreads();
@@ -27,18 +28,27 @@ __global__ void ensemble_finalize_kernel(GswEnsembleArgs a) {
     }
 }
 
+// Wave speed of every member's current state: one warp per brick (a brick belongs to one
+// member), its rows read by the lanes side by side, one atomicMax per brick that exceeds the
+// member's value so far. (An atomicMax and a 64-bit division per cell took 371 us for eight
+// members of 0.9 M active cells.)
 __global__ void __launch_bounds__(256) ensemble_lammax_kernel(GswEnsembleArgs a) {
-    const int64_t BS = (int64_t)a.brick_h * GSW_BRICK_PITCH;
-    const int64_t nslots = a.n_bricks * BS;
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nslots;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        if (!(a.flags[s] & GSW_SLOT_ACTIVE)) continue;
-        const int mi = a.brick_member[s / BS];
-        const GswMember& mb = a.members[mi];
-        const unsigned long long lb = lam_flat_bits(a.q0[s], a.q1[s], a.q2[s], mb.g, mb.h_min, mb.h_min_cfl,
-                                                    mb.linf != 0);
-        if (lb != 0ull) atomicMax((unsigned long long*)&a.states[mi].lam_bits, lb);
+    chain_begin();
+    const int64_t brick = (int64_t)blockIdx.x * blockDim.y + threadIdx.y;
+    if (brick >= a.n_bricks) return;                              // warp-uniform
+    const int mi = a.brick_member[brick];
+    const GswMember& mb = a.members[mi];
+    const int64_t base = brick * a.brick_h * GSW_BRICK_PITCH + threadIdx.x;
+    unsigned long long lam = 0ull;
+    for (int r = 0; r < a.brick_h; ++r) {
+        const int64_t s = base + (int64_t)r * GSW_BRICK_PITCH;
+        const uint8_t f = a.flags[s];
+        const float h = a.q0[s], hu = a.q1[s], hv = a.q2[s];
+        if (!(f & GSW_SLOT_ACTIVE)) continue;
+        const unsigned long long lb = lam_flat_bits(h, hu, hv, mb.g, mb.h_min, mb.h_min_cfl, mb.linf != 0);
+        lam = lb > lam ? lb : lam;
     }
+    warp_max_to(lam, (unsigned long long*)&a.states[mi].lam_bits);
 }
 
 }  // namespace gsw
@@ -63,9 +73,8 @@ extern "C" int gsw_ensemble_lammax(const GswEnsembleArgs* a, void* stream) {
     GSW_CHECK_ABI(a);
     int rc = check_ens(a, false);
     if (rc) return rc;
-    const int64_t nslots = a->n_bricks * (int64_t)a->brick_h * GSW_BRICK_PITCH;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count() * 8, (nslots + 255) / 256));
-    ensemble_lammax_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(*a);
+    if (a->n_bricks == 0) return GSW_OK;
+    launch_chained(ensemble_lammax_kernel, dim3((unsigned)((a->n_bricks + 7) / 8)), dim3(32, 8), (cudaStream_t)stream, *a);
     return check_launch("ensemble_lammax");
 }
 
@@ -73,7 +82,7 @@ extern "C" int gsw_ensemble_finalize(const GswEnsembleArgs* a, void* stream) {
     GSW_CHECK_ABI(a);
     int rc = check_ens(a, false);
     if (rc) return rc;
-    ensemble_finalize_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(*a);
+    launch_chained(ensemble_finalize_kernel, dim3(1), dim3(256), (cudaStream_t)stream, *a);
     return check_launch("ensemble_finalize");
 }
 

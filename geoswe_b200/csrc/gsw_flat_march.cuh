@@ -16,6 +16,7 @@ namespace gsw {
 
 template <typename T, typename I, bool STEP, int REGS, bool REFPOW, bool LEAN>
 __global__ void __maxnreg__(REGS) flat_march_kernel(FlatK<T> p) {
+    chain_begin();
     if (STEP && p.st->done) return;
     const int64_t item = (int64_t)blockIdx.x * blockDim.y + threadIdx.y;   // (brick, row segment)
     const int64_t rel = item / p.segs;
@@ -85,10 +86,10 @@ inline int fill_flat(const GswFlatArgs* a, FlatK<T>& k, bool step) {
 template <bool STEP, bool REFPOW, bool LEAN>
 inline void launch_flat_caps(const FlatK<float>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
     const dim3 b(32, W);
-    if (STEP && mb == 3) flat_march_kernel<float, int, STEP, STEP ? 96 : 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
-    else if (STEP && mb == 4) flat_march_kernel<float, int, STEP, STEP ? 64 : 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
-    else if (STEP && mb == 5) flat_march_kernel<float, int, STEP, STEP ? 72 : 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
-    else flat_march_kernel<float, int, STEP, 80, REFPOW, LEAN><<<blocks, b, 0, s>>>(k);
+    if (STEP && mb == 3) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 96 : 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
+    else if (STEP && mb == 4) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 64 : 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
+    else if (STEP && mb == 5) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 72 : 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
+    else launch_chained(flat_march_kernel<float, int, STEP, 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
 }
 
 // The production configuration (the LEAN kernel: rain none or uniform, quadratic
@@ -98,13 +99,13 @@ inline void launch_flat_shape(const FlatK<float>& k, int mb, unsigned blocks, in
     const bool lean = k.ph.rain_kind != GSW_RAIN_GRIDDED && k.ph.rain_kind != GSW_RAIN_LOOKUP &&
                       k.ph.quad != 0 && k.ph.keep_h != 0 && k.ph.linf == 0;
     if ((k.m.nb + 1) * (int64_t)k.m.bh * GSW_BRICK_PITCH > INT32_MAX)
-        flat_march_kernel<float, int64_t, STEP, 128, REFPOW, false><<<blocks, dim3(32, W), 0, s>>>(k);
+        launch_chained(flat_march_kernel<float, int64_t, STEP, 128, REFPOW, false>, dim3(blocks), dim3(32, W), s, k);
     else if (STEP && lean) launch_flat_caps<STEP, REFPOW, STEP>(k, mb, blocks, W, s);
     else launch_flat_caps<STEP, REFPOW, false>(k, mb, blocks, W, s);
 }
 template <bool STEP, bool REFPOW>
 inline void launch_flat_shape(const FlatK<double>& k, int, unsigned blocks, int W, cudaStream_t s) {
-    flat_march_kernel<double, int64_t, STEP, 200, false, false><<<blocks, dim3(32, W), 0, s>>>(k);
+    launch_chained(flat_march_kernel<double, int64_t, STEP, 200, false, false>, dim3(blocks), dim3(32, W), s, k);
 }
 
 template <typename T, bool STEP>

@@ -11,16 +11,22 @@ namespace gsw {
 
 template <typename T>
 __global__ void inflow_kernel(GswInflowArgs a) {
+    chain_begin();
     if (a.state->done) return;
     T* q0 = (T*)a.q0; T* q1 = (T*)a.q1; T* q2 = (T*)a.q2;
     const T* bed = (const T*)a.bed;
     __shared__ double s_Q, s_sum, s_add;
     __shared__ T s_zmin, s_zmax;
     __shared__ int s_wet, s_nlow, s_flat;
+    // the discharge by another warp while the depths are added; a dry inlet needs it in thread 0
+    if (threadIdx.x == 32) s_Q = np_interp(a.state->t, a.t_knots, a.q_knots, a.n_knots);
+    const T own = a.hsum != nullptr ? (T)0 : block_pairwise_sum<T>(q0, a.inlet_off, a.n);
     if (threadIdx.x == 0) {
-        s_Q = np_interp(a.state->t, a.t_knots, a.q_knots, a.n_knots);
-        s_sum = a.hsum != nullptr ? *a.hsum : (double)pairwise_sum<T>(q0, a.inlet_off, 0, a.n);
+        s_sum = a.hsum != nullptr ? *a.hsum : (double)own;
         s_wet = s_sum > 0.0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
         if (!s_wet) {
             T zmin = bed[a.inlet_off[0]], zmax = zmin;
             for (int k = 1; k < a.n; ++k) {
@@ -84,12 +90,14 @@ __global__ void inflow_kernel(GswInflowArgs a) {
 // This rank's share of an inlet's depth sum (a split run all-reduces these).
 template <typename T>
 __global__ void inflow_depth_sum_kernel(GswInflowArgs a, double* out) {
+    chain_begin();
     if (threadIdx.x == 0)
         *out = a.n > 0 ? (double)pairwise_sum<T>((const T*)a.q0, a.inlet_off, 0, a.n) : 0.0;
 }
 
 template <typename T>
 __global__ void flat_inflow_depth_sum_kernel(GswFlatInflowArgs a, double* out) {
+    chain_begin();
     if (threadIdx.x == 0)
         *out = a.n > 0 ? (double)pairwise_sum<T>((const T*)a.q0, a.nbr_slot, 0, a.n) : 0.0;
 }
@@ -98,16 +106,22 @@ __global__ void flat_inflow_depth_sum_kernel(GswFlatInflowArgs a, double* out) {
 // inlet; thread 0 evaluates Q, the depth sum and the dry seed, all threads write ghosts.
 template <typename T>
 __global__ void flat_inflow_kernel(GswFlatInflowArgs a) {
+    chain_begin();
     if (a.state->done) return;
     T* q0 = (T*)a.q0; T* q1 = (T*)a.q1; T* q2 = (T*)a.q2;
     const T* bed = (const T*)a.bed;
     __shared__ double s_Q, s_sum, s_zmin, s_add, s_nlow;
     __shared__ T s_seed;
     __shared__ int s_wet, s_flat;
+    // the discharge by another warp while the depths are added; a dry inlet needs it in thread 0
+    if (threadIdx.x == 32) s_Q = np_interp(a.state->t, a.t_knots, a.q_knots, a.n_knots);
+    const T own = a.hsum != nullptr ? (T)0 : block_pairwise_sum<T>(q0, a.nbr_slot, a.n);
     if (threadIdx.x == 0) {
-        s_Q = np_interp(a.state->t, a.t_knots, a.q_knots, a.n_knots);
-        s_sum = a.hsum != nullptr ? *a.hsum : (double)pairwise_sum<T>(q0, a.nbr_slot, 0, a.n);
+        s_sum = a.hsum != nullptr ? *a.hsum : (double)own;
         s_wet = s_sum > 0.0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
         if (!s_wet && a.dry != nullptr) {       // the seed's reductions over every rank's cells
             const double zlo = a.dry[0], zhi = a.dry[1];
             s_seed = (T)__dadd_rn(zlo, __dmul_rn(0.10, __dsub_rn(zhi, zlo)));
@@ -172,6 +186,7 @@ __global__ void flat_inflow_kernel(GswFlatInflowArgs a) {
 // the on-device stage interpolation of :2338-2350). One thread per ring cell.
 template <typename T>
 __global__ void flat_ring_kernel(GswFlatRingArgs a) {
+    chain_begin();
     if (a.state->done) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
@@ -204,24 +219,28 @@ __global__ void flat_ring_kernel(GswFlatRingArgs a) {
 
 // ---- per-step forcings of the flat loop (compressed_solver.py:2330-2366) ----
 // Landcover infiltration, infiltrate_flat (:143-158).
-__global__ void flat_infiltrate_kernel(GswFlatForcingArgs a) {
+// A thread per slot, every load issued before the first test: the pass is latency (its state
+// sits in L2 on meshes that take forcings), not bytes.
+__global__ void __launch_bounds__(256) flat_infiltrate_kernel(GswFlatForcingArgs a) {
+    chain_begin();
     if (a.state->done) return;
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= a.nslots) return;
     const float dt = a.state->dt_f32;
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.nslots;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        if (!(a.flags[k] & GSW_SLOT_ACTIVE)) continue;
-        const float h = a.q0[k];
-        if (h < a.h_min) continue;
-        const float dh = a.infil_tab[a.n_cls ? a.n_cls[k] : 0] * dt;
-        float hn = h - dh;
-        if (hn < 0.0f) hn = 0.0f;
-        const float r = hn / h;
-        a.q0[k] = hn; a.q1[k] = a.q1[k] * r; a.q2[k] = a.q2[k] * r;
-    }
+    const uint8_t f = a.flags[k];
+    const float h = a.q0[k], hu = a.q1[k], hv = a.q2[k];
+    const uint8_t c = a.n_cls ? a.n_cls[k] : 0;
+    if (!(f & GSW_SLOT_ACTIVE) || h < a.h_min) return;
+    const float dh = a.infil_tab[c] * dt;
+    float hn = h - dh;
+    if (hn < 0.0f) hn = 0.0f;
+    const float r = hn / h;
+    a.q0[k] = hn; a.q1[k] = hu * r; a.q2[k] = hv * r;
 }
 
 // Open-boundary sponge over its band, sponge_band (:1320-1328).
 __global__ void flat_sponge_kernel(GswFlatForcingArgs a) {
+    chain_begin();
     if (a.state->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.sp_n) return;
@@ -234,62 +253,66 @@ __global__ void flat_sponge_kernel(GswFlatForcingArgs a) {
 
 // Green-Ampt infiltration and the linear-reservoir drain, ga_drain_flat / ga_flat /
 // drain_tau_flat (:313-420): one momentum scale accumulated over both, as the reference.
-__global__ void flat_ga_drain_kernel(GswFlatForcingArgs a) {
+// A thread per slot, as flat_infiltrate_kernel.
+__global__ void __launch_bounds__(256) flat_ga_drain_kernel(GswFlatForcingArgs a) {
+    chain_begin();
     if (a.state->done) return;
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= a.nslots) return;
     const float dt = a.state->dt_f32;
     const bool ga = a.ga_mode == 1 || a.ga_mode == 2;
     const bool drain = a.ga_mode == 1 || a.ga_mode == 3;
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.nslots;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        if (!(a.flags[k] & GSW_SLOT_ACTIVE)) continue;
-        float h = a.q0[k];
-        if (h <= 0.0f) continue;
-        float scale = 1.0f;
-        if (ga) {
-            const int c = a.ga_cls[k];
-            const float K = a.Ks_t[c];
-            if (K > 0.0f) {
-                const float KsDt = K * dt;
-                const float head = a.psi_t[c] + h;
-                const float F0 = a.F[k];
-                const float A = F0 + KsDt;
-                const float disc = A * A + 4.0f * KsDt * head * a.dth_t[c];
-                const float F1 = 0.5f * (A + sqrtf(fmaxf(disc, 0.0f)));
-                const float dF_raw = F1 - F0;
-                float dF = (dF_raw > 0.0f) ? dF_raw : 0.0f;
-                if (dF > h) dF = h;
-                const float room = (a.Fmax ? a.Fmax[k] : 3.0e38f) - F0;
-                if (dF > room) dF = (room > 0.0f) ? room : 0.0f;
-                const float hn = h - dF;
-                if (drain) {
-                    scale = scale * (hn / h);
-                } else {
-                    scale = hn / h;
-                }
-                h = hn;
-                a.F[k] = F0 + dF;
-            } else if (!drain) {
-                continue;
+    const uint8_t f = a.flags[k];
+    float h = a.q0[k];
+    const float hu = a.q1[k], hv = a.q2[k];
+    const int c = ga ? a.ga_cls[k] : 0;
+    const float F0 = ga ? a.F[k] : 0.0f;
+    const float Fmax = ga && a.Fmax ? a.Fmax[k] : 3.0e38f;
+    const float it = drain ? a.inv_tau[k] : 0.0f;
+    if (!(f & GSW_SLOT_ACTIVE) || h <= 0.0f) return;
+    float scale = 1.0f;
+    if (ga) {
+        const float K = a.Ks_t[c];
+        if (K > 0.0f) {
+            const float KsDt = K * dt;
+            const float head = a.psi_t[c] + h;
+            const float A = F0 + KsDt;
+            const float disc = A * A + 4.0f * KsDt * head * a.dth_t[c];
+            const float F1 = 0.5f * (A + sqrtf(fmaxf(disc, 0.0f)));
+            const float dF_raw = F1 - F0;
+            float dF = (dF_raw > 0.0f) ? dF_raw : 0.0f;
+            if (dF > h) dF = h;
+            const float room = Fmax - F0;
+            if (dF > room) dF = (room > 0.0f) ? room : 0.0f;
+            const float hn = h - dF;
+            if (drain) {
+                scale = scale * (hn / h);
+            } else {
+                scale = hn / h;
             }
+            h = hn;
+            a.F[k] = F0 + dF;
+        } else if (!drain) {
+            return;
         }
-        if (drain) {
-            const float it = a.inv_tau[k];
-            if (it > 0.0f && h > 0.0f) {
-                const float decay = __expf(-dt * it);
-                scale = scale * decay;
-                h = h * decay;
-            } else if (!ga) {
-                continue;
-            }
-        }
-        a.q0[k] = h;
-        a.q1[k] = a.q1[k] * scale;
-        a.q2[k] = a.q2[k] * scale;
     }
+    if (drain) {
+        if (it > 0.0f && h > 0.0f) {
+            const float decay = __expf(-dt * it);
+            scale = scale * decay;
+            h = h * decay;
+        } else if (!ga) {
+            return;
+        }
+    }
+    a.q0[k] = h;
+    a.q1[k] = hu * scale;
+    a.q2[k] = hv * scale;
 }
 
 // Stage clamp, stage_clamp_flat (:422-437), then the karst drain cap, drain_cap (:268-283).
 __global__ void flat_clamp_kernel(GswFlatForcingArgs a, bool cap) {
+    chain_begin();
     if (a.state->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = cap ? a.dr_n : a.cl_n;
@@ -317,8 +340,8 @@ extern "C" int gsw_inflow_apply(const GswInflowArgs* a, void* stream) {
         a->n_knots < 1 || !a->state || a->ngh < 1)
         return set_error(GSW_ERR_INVALID, "inflow: null pointer or empty hydrograph");
     cudaStream_t s = (cudaStream_t)stream;
-    if (a->dtype == GSW_F32) inflow_kernel<float><<<1, 256, 0, s>>>(*a);
-    else if (a->dtype == GSW_F64) inflow_kernel<double><<<1, 256, 0, s>>>(*a);
+    if (a->dtype == GSW_F32) launch_chained(inflow_kernel<float>, dim3(1), dim3(256), s, *a);
+    else if (a->dtype == GSW_F64) launch_chained(inflow_kernel<double>, dim3(1), dim3(256), s, *a);
     else return set_error(GSW_ERR_INVALID, "inflow: bad dtype");
     return check_launch("inflow");
 }
@@ -328,8 +351,8 @@ extern "C" int gsw_inflow_depth_sum(const GswInflowArgs* a, double* out, void* s
     if (!out || !a->q0 || (a->n > 0 && !a->inlet_off) || a->n < 0)
         return set_error(GSW_ERR_INVALID, "inflow depth sum: null pointer or negative count");
     cudaStream_t s = (cudaStream_t)stream;
-    if (a->dtype == GSW_F32) inflow_depth_sum_kernel<float><<<1, 32, 0, s>>>(*a, out);
-    else if (a->dtype == GSW_F64) inflow_depth_sum_kernel<double><<<1, 32, 0, s>>>(*a, out);
+    if (a->dtype == GSW_F32) launch_chained(inflow_depth_sum_kernel<float>, dim3(1), dim3(32), s, *a, out);
+    else if (a->dtype == GSW_F64) launch_chained(inflow_depth_sum_kernel<double>, dim3(1), dim3(32), s, *a, out);
     else return set_error(GSW_ERR_INVALID, "inflow depth sum: bad dtype");
     return check_launch("inflow_depth_sum");
 }
@@ -339,8 +362,8 @@ extern "C" int gsw_flat_inflow_depth_sum(const GswFlatInflowArgs* a, double* out
     if (!out || !a->q0 || (a->n > 0 && !a->nbr_slot) || a->n < 0)
         return set_error(GSW_ERR_INVALID, "flat inflow depth sum: null pointer or negative count");
     cudaStream_t s = (cudaStream_t)stream;
-    if (a->dtype == GSW_F32) flat_inflow_depth_sum_kernel<float><<<1, 32, 0, s>>>(*a, out);
-    else if (a->dtype == GSW_F64) flat_inflow_depth_sum_kernel<double><<<1, 32, 0, s>>>(*a, out);
+    if (a->dtype == GSW_F32) launch_chained(flat_inflow_depth_sum_kernel<float>, dim3(1), dim3(32), s, *a, out);
+    else if (a->dtype == GSW_F64) launch_chained(flat_inflow_depth_sum_kernel<double>, dim3(1), dim3(32), s, *a, out);
     else return set_error(GSW_ERR_INVALID, "flat inflow depth sum: bad dtype");
     return check_launch("flat_inflow_depth_sum");
 }
@@ -352,8 +375,8 @@ extern "C" int gsw_flat_inflow_apply(const GswFlatInflowArgs* a, void* stream) {
         !a->q_knots || a->n_knots < 1 || !a->state || !(a->ds > 0.0))
         return set_error(GSW_ERR_INVALID, "flat inflow: null pointer, empty hydrograph or ds <= 0");
     cudaStream_t s = (cudaStream_t)stream;
-    if (a->dtype == GSW_F32) flat_inflow_kernel<float><<<1, 256, 0, s>>>(*a);
-    else if (a->dtype == GSW_F64) flat_inflow_kernel<double><<<1, 256, 0, s>>>(*a);
+    if (a->dtype == GSW_F32) launch_chained(flat_inflow_kernel<float>, dim3(1), dim3(256), s, *a);
+    else if (a->dtype == GSW_F64) launch_chained(flat_inflow_kernel<double>, dim3(1), dim3(256), s, *a);
     else return set_error(GSW_ERR_INVALID, "flat inflow: bad dtype");
     return check_launch("flat_inflow");
 }
@@ -366,8 +389,8 @@ extern "C" int gsw_flat_ring_stage(const GswFlatRingArgs* a, void* stream) {
         return set_error(GSW_ERR_INVALID, "ring stage: null pointer, NG < 1 or fewer than 2 stage times");
     cudaStream_t s = (cudaStream_t)stream;
     const int grid = (a->n + 255) / 256;
-    if (a->dtype == GSW_F32) flat_ring_kernel<float><<<grid, 256, 0, s>>>(*a);
-    else if (a->dtype == GSW_F64) flat_ring_kernel<double><<<grid, 256, 0, s>>>(*a);
+    if (a->dtype == GSW_F32) launch_chained(flat_ring_kernel<float>, dim3(grid), dim3(256), s, *a);
+    else if (a->dtype == GSW_F64) launch_chained(flat_ring_kernel<double>, dim3(grid), dim3(256), s, *a);
     else return set_error(GSW_ERR_INVALID, "ring stage: bad dtype");
     return check_launch("flat_ring");
 }
@@ -377,15 +400,17 @@ extern "C" int gsw_flat_forcings(const GswFlatForcingArgs* a, void* stream) {
     if (!a->q0 || !a->q1 || !a->q2 || !a->flags || !a->state || a->nslots < 0)
         return set_error(GSW_ERR_INVALID, "flat forcings: null state or flags");
     cudaStream_t s = (cudaStream_t)stream;
-    const int grid_all = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count() * 8, (a->nslots + 255) / 256));
+    const int64_t all = std::max<int64_t>(1, (a->nslots + 255) / 256);
+    if (all > 0x7fffffffLL) return set_error(GSW_ERR_INVALID, "flat forcings: too many slots");
+    const unsigned grid_all = (unsigned)all;
     if (a->phase == 0) {
         if (a->infil_tab) {
-            flat_infiltrate_kernel<<<grid_all, 256, 0, s>>>(*a);
+            launch_chained(flat_infiltrate_kernel, dim3(grid_all), dim3(256), s, *a);
             if (int rc = check_launch("flat_infiltrate")) return rc;
         }
         if (a->sp_n > 0) {
             if (!a->sp_slots || !a->sp_keep || !a->sp_amb) return set_error(GSW_ERR_INVALID, "sponge: null arrays");
-            flat_sponge_kernel<<<(a->sp_n + 255) / 256, 256, 0, s>>>(*a);
+            launch_chained(flat_sponge_kernel, dim3((a->sp_n + 255) / 256), dim3(256), s, *a);
             if (int rc = check_launch("flat_sponge")) return rc;
         }
         return GSW_OK;
@@ -396,17 +421,17 @@ extern "C" int gsw_flat_forcings(const GswFlatForcingArgs* a, void* stream) {
         if ((a->ga_mode != 3 && (!a->ga_cls || !a->Ks_t || !a->psi_t || !a->dth_t || !a->F)) ||
             (a->ga_mode != 2 && !a->inv_tau))
             return set_error(GSW_ERR_INVALID, "Green-Ampt / drain: null arrays");
-        flat_ga_drain_kernel<<<grid_all, 256, 0, s>>>(*a);
+        launch_chained(flat_ga_drain_kernel, dim3(grid_all), dim3(256), s, *a);
         if (int rc = check_launch("flat_ga_drain")) return rc;
     }
     if (a->cl_n > 0) {
         if (!a->cl_slots || !a->cl_hmax) return set_error(GSW_ERR_INVALID, "stage clamp: null arrays");
-        flat_clamp_kernel<<<(a->cl_n + 63) / 64, 64, 0, s>>>(*a, false);
+        launch_chained(flat_clamp_kernel, dim3((a->cl_n + 63) / 64), dim3(64), s, *a, false);
         if (int rc = check_launch("flat_clamp")) return rc;
     }
     if (a->dr_n > 0) {
         if (!a->dr_slots || !a->dr_htgt) return set_error(GSW_ERR_INVALID, "drain cap: null arrays");
-        flat_clamp_kernel<<<(a->dr_n + 255) / 256, 256, 0, s>>>(*a, true);
+        launch_chained(flat_clamp_kernel, dim3((a->dr_n + 255) / 256), dim3(256), s, *a, true);
         if (int rc = check_launch("flat_drain_cap")) return rc;
     }
     return GSW_OK;

@@ -86,14 +86,15 @@ float div_const_recip(float g) {
 
 namespace gsw {
 
-__global__ void dt_finalize_kernel(GswDtParams p, GswLoopState* s) { dt_finalize_one(p, s, s->lam_bits); }
+__global__ void dt_finalize_kernel(GswDtParams p, GswLoopState* s) { chain_begin(); dt_finalize_one(p, s, s->lam_bits); }
 // The same with the parameters read from device memory: a captured launch then follows
 // whatever t_end / dt_max / max_steps the last gsw_dt_params_upload wrote.
 __global__ void dt_finalize_dev_kernel(const GswDtParams* p, GswLoopState* s) {
+    chain_begin();
     dt_finalize_one(*p, s, s->lam_bits);
 }
 
-__global__ void loop_commit_kernel(GswLoopState* s) { loop_commit(s); }
+__global__ void loop_commit_kernel(GswLoopState* s) { chain_begin(); loop_commit(s); }
 
 }  // namespace gsw
 
@@ -112,7 +113,7 @@ extern "C" int gsw_dt_finalize(const GswDtParams* p, GswLoopState* state, void* 
     GSW_CHECK_ABI(p);
     if (!state) return set_error(GSW_ERR_INVALID, "dt_finalize: null state");
     if (int rc = check_dt_params(p)) return rc;
-    dt_finalize_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(*p, state);
+    launch_chained(dt_finalize_kernel, dim3(1), dim3(1), (cudaStream_t)stream, *p, state);
     return check_launch("dt_finalize");
 }
 
@@ -129,13 +130,13 @@ extern "C" int gsw_dt_params_upload(const GswDtParams* p, GswDtParams* dev, void
 
 extern "C" int gsw_dt_finalize_dev(const GswDtParams* dev, GswLoopState* state, void* stream) {
     if (!dev || !state) return set_error(GSW_ERR_INVALID, "dt_finalize_dev: null pointer");
-    dt_finalize_dev_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(dev, state);
+    launch_chained(dt_finalize_dev_kernel, dim3(1), dim3(1), (cudaStream_t)stream, dev, state);
     return check_launch("dt_finalize_dev");
 }
 
 extern "C" int gsw_loop_commit(GswLoopState* state, void* stream) {
     if (!state) return set_error(GSW_ERR_INVALID, "loop_commit: null state");
-    loop_commit_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(state);
+    launch_chained(loop_commit_kernel, dim3(1), dim3(1), (cudaStream_t)stream, state);
     return check_launch("loop_commit");
 }
 

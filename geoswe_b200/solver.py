@@ -587,7 +587,7 @@ class Solver2D:
         src, dst = self._buf[k_parity], self._buf[1 - k_parity]
         s = _stream()
         L.call("gsw_bc_fill", C.byref(self._bc_args(src)), s)
-        n = 2 + 2 * len(T.stages) + (1 if len(T.stages) > 1 else 0)
+        n = 2 + len(T.stages) + (1 if len(T.stages) > 1 else 0)
         n += self._apply_inflows(T, src, s)
         windows = self._overlap_windows() if self.halo is not None else None
         if windows is None:
