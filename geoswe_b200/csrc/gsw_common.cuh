@@ -37,11 +37,23 @@ using gsw_rt::sm_count;
 using gsw_rt::count_launch;
 using gsw_rt::div_const_recip;
 
-// Launch of a kernel of the time loop, and what each of them does first.
-__device__ __forceinline__ void chain_begin() {}
+// Kernels of the time loop are launched as programmatic dependents of the kernel before them in
+// the stream: a step of a small grid is several short kernels, and the next one's launch then
+// overlaps the one that runs. Each of them calls chain_begin() before it touches memory: it
+// waits until every kernel before it has completed and its writes are visible (each waits for
+// its own predecessor, so the order is the stream's), then lets the next one be launched.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 template <class... P, class... A>
 inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
-    kernel<<<grid, block, 0, s>>>(std::forward<A>(args)...);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid; c.blockDim = block; c.stream = s; c.attrs = at; c.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);        // check_launch reads the error
 }
 
 // Max of a non-negative IEEE-bits value over the block, then one atomicMax.
