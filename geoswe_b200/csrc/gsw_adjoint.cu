@@ -77,6 +77,51 @@ __device__ __forceinline__ void load_state(const FlatMesh<T>& m, int64_t s, Cell
 }
 
 // ---------------------------------------------------------------------------- A
+// One row of kernel A in binary32: the update run backwards from the row's old depth and
+// residual, which march_rows recomputes as the forward step did.
+struct AdjTailRow {
+    const AdjK<float>& p;
+    double* s_nbar;
+    int64_t base;                    // the lane's slot of row r0
+    int bi, bj, r0, lane;
+    float dt, rate;
+    const float* frame;
+    bool out_lane;
+    double rate_acc = 0.0;
+    __device__ __forceinline__ void pre(int) {}
+    __device__ __forceinline__ void row(int k, float h, float rh, float rhu, float rhv) {
+        if (!out_lane) return;
+        const FlatMesh<float>& m = p.m;
+        const FlatPhys<float>& ph = p.ph;
+        const int64_t o = base + (int64_t)k * GSW_BRICK_PITCH;
+        const uint8_t f = m.flags[o];
+        if (f & GSW_SLOT_ACTIVE) {
+            if (ph.rain_kind == GSW_RAIN_UNIFORM) rh = rh + rate;
+            else if (ph.rain_kind == GSW_RAIN_GRIDDED) {
+                const int i = bi * m.bh + r0 + k, j = bj * GSW_BRICK_W + (lane - 1);
+                rh = rh + frame[(int64_t)(i - ph.ngh) * ph.ny + (j - ph.ngh)];
+            }
+            const float h1 = h + dt * rh;
+            const float hu1 = __ldg(m.q1 + o) + dt * rhu;
+            const float hv1 = __ldg(m.q2 + o) + dt * rhv;
+            const int cls = m.ncls ? (int)m.ncls[o] : 0;
+            const float n = ph.ntab[cls];
+            const Bar3<float> out_b = load_bar(p.li0, p.li1, p.li2, o);
+            Bar3<float> in_b;
+            float n_b;
+            wetdry_friction_bwd<float>(h1, hu1, hv1, n, dt, ph.g, ph.h_min, ph.vcap, ph.quad != 0, ph.keep_h != 0,
+                                       ph.ref_pow != 0, out_b, in_b, n_b);
+            p.lo0[o] = in_b.h; p.lo1[o] = in_b.hu; p.lo2[o] = in_b.hv;
+            p.rb0[o] = dt * in_b.h; p.rb1[o] = dt * in_b.hu; p.rb2[o] = dt * in_b.hv;
+            if (ph.rain_kind == GSW_RAIN_UNIFORM) rate_acc += (double)(dt * in_b.h);
+            if (n_b != 0.0f && cls < p.n_tab_len) atomicAdd(&s_nbar[cls], (double)n_b);
+        } else if (f & GSW_SLOT_STORED) {
+            p.lo0[o] = 0.0f; p.lo1[o] = 0.0f; p.lo2[o] = 0.0f;
+            p.rb0[o] = 0.0f; p.rb1[o] = 0.0f; p.rb2[o] = 0.0f;
+        }
+    }
+};
+
 template <typename T, int MINB>
 __global__ void __launch_bounds__(128, MINB) adj_tail_kernel(AdjK<T> p) {
     chain_begin();
@@ -98,7 +143,17 @@ __global__ void __launch_bounds__(128, MINB) adj_tail_kernel(AdjK<T> p) {
     const T* frame = nullptr;
     if (ph.rain_kind == GSW_RAIN_UNIFORM) rate = ph.rain[p.st->rain_idx];
     if (ph.rain_kind == GSW_RAIN_GRIDDED) frame = ph.rain + (int64_t)p.st->rain_idx * ph.nx * ph.ny;
-    if (bidx < m.nb) {
+    if constexpr (sizeof(T) == 4) {
+        if (bidx < m.nb) {
+            const BrickView v = brick_view(m, bidx);
+            const int r0 = seg * m.bh / p.segs, r1 = (seg + 1) * m.bh / p.segs;
+            const FlatRows<int64_t> acc = flat_rows<int64_t>(m, v, r0, lane);
+            AdjTailRow upd = {p, s_nbar, bidx * v.BS + (int64_t)r0 * GSW_BRICK_PITCH + (lane - 1), m.bij[2 * bidx],
+                              m.bij[2 * bidx + 1], r0, lane, dt, rate, frame, lane >= 1 && lane <= 30};
+            march_rows(acc, upd, r1 - r0, face_phys(ph), !face_ranges(ph.g, ph.h_min, ph.h_min));
+            rate_acc = upd.rate_acc;
+        }
+    } else if (bidx < m.nb) {
         const BrickView v = brick_view(m, bidx);
         const int bi = m.bij[2 * bidx], bj = m.bij[2 * bidx + 1];
         const int bh = m.bh;

@@ -108,6 +108,11 @@ __device__ __forceinline__ Face<T> shfl_up_face(const Face<T>& f) {
     return r;
 }
 
+__device__ __forceinline__ FacePhys face_phys(const FlatPhys<float>& ph) {
+    return {ph.inv_dx, ph.inv_dy, 0.5f * ph.inv_dx, 0.5f * ph.inv_dy, ph.half_dx, ph.half_dy,
+            ph.g, ph.g_recip != 0.0f ? ph.g_recip : rcp_in(ph.g), ph.h_min};
+}
+
 // Slots of one lane's rows of a brick, as BrickView::slot, by one base per row range. I: the
 // slots' integer type, 32-bit where the mesh has fewer than 2^31 slots (a 64-bit base costs
 // registers and address arithmetic on every access), else 64-bit.
@@ -339,9 +344,7 @@ __device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, c
         const bool general = !face_ranges(ph.g, ph.h_min, ph.h_min_cfl) || ph.h_min_cfl != ph.h_min;
         FlatRow<I, STEP, REFPOW, LEAN> upd = {m, ph, (I)(bidx * v.BS) + (lane - 1), bi, bj, r0, lane, dt, rate, frame, general,
                                            lane >= 1 && lane <= 30};
-        const FacePhys fp = {ph.inv_dx, ph.inv_dy, 0.5f * ph.inv_dx, 0.5f * ph.inv_dy, ph.half_dx, ph.half_dy,
-                             ph.g, ph.g_recip != 0.0f ? ph.g_recip : rcp_in(ph.g), ph.h_min};
-        march_rows(acc, upd, r1 - r0, fp, general);
+        march_rows(acc, upd, r1 - r0, face_phys(ph), general);
         const unsigned long long l = lam_bits_of32(upd.lam32);
         return LEAN || l > upd.lam64 ? l : upd.lam64;
     } else {
