@@ -333,17 +333,32 @@ class FlatAdjoint:
         a.state = _ptr(self._state)
         return a
 
-    def _one_step(self, src, dst, p, record):
-        s = _stream()
-        L.call("gsw_dt_finalize", C.byref(p), _ptr(self._state), s)
-        if self.inlet is not None:
-            L.call("gsw_flat_inflow_apply", C.byref(self._inflow_args(src)), s)
-        L.call("gsw_flat_step", C.byref(self._flat_args(src, dst)), s)
-        n = 2 + (self.inlet is not None)
-        if record and self.G:
-            L.call("gsw_gauge_record", C.byref(self._gauge_args(dst[0], 1)), s)
-            n += 1
-        self.kernel_launches += n
+    def _stepper(self, p, record):
+        """Launcher of one step from buffer k to buffer 1 - k: the argument structs of both
+        directions are filled once per pass (their buffers belong to this object and the
+        pass's parameters to the caller's frame), so a step on the host is its launches."""
+        lib, s, n_launch = L.lib(), _stream(), 2 + (self.inlet is not None) + bool(record and self.G)
+        keep, dirs = [p], []
+        for k in (0, 1):
+            src, dst = self._buf[k], self._buf[1 - k]
+            args = [(lib.gsw_dt_finalize, (C.byref(p), _ptr(self._state), s))]
+            flat, inflow, gauge = self._flat_args(src, dst), None, None
+            if self.inlet is not None:
+                inflow = self._inflow_args(src)
+                args.append((lib.gsw_flat_inflow_apply, (C.byref(inflow), s)))
+            args.append((lib.gsw_flat_step, (C.byref(flat), s)))
+            if record and self.G:
+                gauge = self._gauge_args(dst[0], 1)
+                args.append((lib.gsw_gauge_record, (C.byref(gauge), s)))
+            keep += [flat, inflow, gauge]
+            dirs.append(args)
+
+        def step(k, _keep=keep):
+            for fn, a in dirs[k]:
+                if fn(*a) != L.OK:
+                    raise L.GswError(fn.__name__, -1, lib.gsw_last_error().decode(errors="replace"))
+            self.kernel_launches += n_launch
+        return step
 
     # ----------------------------------------------------------------- forward
     def forward(self, *, replay=False, snapshots=True):
@@ -364,10 +379,10 @@ class FlatAdjoint:
             self.dt_tab.zero_()
             L.call("gsw_flat_lammax", C.byref(self._flat_args(self._buf[0])),
                    C.c_void_p(self._state.data_ptr() + L.GswLoopState.lam_bits.offset), _stream())
-        p = self._dt_params(2 if replay else 0)
+        step = self._stepper(self._dt_params(2 if replay else 0), True)
         cur = 0
         for n in range(self.N):
-            self._one_step(self._buf[cur], self._buf[1 - cur], p, True)
+            step(cur)
             cur = 1 - cur
             if (n + 1) in chain:
                 self._snaps[n + 1] = [x.clone() for x in self._buf[cur]]
@@ -424,6 +439,8 @@ class FlatAdjoint:
                                                                  lam0=self._lam[1][0], target=tgt)), _stream())
         work = self._buf
         self._cur = 0
+        step = self._stepper(p2, False)
+        reverse_step = self._reverser(p2)
 
         def restore(n):
             src = self.q_init if n == 0 else self._snaps[n]
@@ -448,7 +465,7 @@ class FlatAdjoint:
             e = events() if timing else None
             self._set_state_n(n0)
             for _ in range(n0, n1):
-                self._one_step(work[self._cur], work[1 - self._cur], p2, False)
+                step(self._cur)
                 self._cur = 1 - self._cur
             if timing:
                 e[1].record()
@@ -456,7 +473,7 @@ class FlatAdjoint:
 
         def reverse(n):
             e = events() if timing else None
-            self._reverse_step(n, work[self._cur], p2)
+            reverse_step(n, self._cur)
             if timing:
                 e[1].record()
                 ev_rev.append(e)
@@ -481,33 +498,63 @@ class FlatAdjoint:
             g_k = torch.from_numpy(interp_weights(self._t_tab[: self.N], np.asarray(self.inlet.t_knots)).T @ qb)
         return g_n, g_s, g_k
 
-    def _reverse_step(self, n, q, p2):
-        """lam_n from lam_{n+1} for state q = q_n (its inlet ghosts are rewritten here)."""
-        s = _stream()
-        self._set_state_n(n)
-        L.call("gsw_dt_finalize", C.byref(p2), _ptr(self._state), s)
-        if self.inlet is not None:
-            L.call("gsw_flat_inflow_apply", C.byref(self._inflow_args(q)), s)
-        a = L.GswFlatAdjArgs()
-        a.abi_version = L.ABI_VERSION
-        a.min_blocks = self.adj_min_blocks if self.code == L.F32 else 0
-        a.f = self._flat_args(q)
-        lin, lout = self._lam[1], self._lam[0]
-        a.lam_in0, a.lam_in1, a.lam_in2 = _ptr(lin[0]), _ptr(lin[1]), _ptr(lin[2])
-        a.lam_out0, a.lam_out1, a.lam_out2 = _ptr(lout[0]), _ptr(lout[1]), _ptr(lout[2])
-        a.rbar0, a.rbar1, a.rbar2 = _ptr(self._rbar[0]), _ptr(self._rbar[1]), _ptr(self._rbar[2])
-        a.n_bar, a.rate_bar = _ptr(self.n_bar), _ptr(self.rate_bar)
-        L.call("gsw_adj_flat_step", C.byref(a), s)
-        k = 3
-        if self.inlet is not None:
-            L.call("gsw_adj_flat_inflow", C.byref(self._inflow_args(q)), _ptr(lout[0]), _ptr(lout[1]),
-                   _ptr(lout[2]), _ptr(self.q_bar), s)
-            k += 2
-        if self.G:
-            L.call("gsw_gauge_adjoint", C.byref(self._gauge_args(q[0], 0, lam0=lout[0], target=self._tgt)), s)
-            k += 1
-        self.kernel_launches += k
-        self._lam = [lin, lout]
+    def _reverser(self, p2):
+        """Launcher of a reverse step: lam_n from lam_{n+1} for the state q_n in buffer k (its
+        inlet ghosts are rewritten here). The loop state of step n (t_n, n) is row n of one
+        device table, uploaded once per sweep: each row is used by its own step alone. The
+        argument structs are filled once per sweep, as in _stepper; a step only points them at
+        its row."""
+        lib, s, G = L.lib(), _stream(), bool(self.G)
+        rows = self._state_tab.to(self.dev, non_blocking=True)
+        row0, lam_off = rows.data_ptr(), L.GswLoopState.lam_bits.offset
+        n_launch = 3 + 2 * (self.inlet is not None) + G
+        made = {}
+
+        def build(k, lin, lout):
+            q = self._buf[k]
+            a = L.GswFlatAdjArgs()
+            a.abi_version = L.ABI_VERSION
+            a.min_blocks = self.adj_min_blocks if self.code == L.F32 else 0
+            a.f = self._flat_args(q)
+            a.lam_in0, a.lam_in1, a.lam_in2 = _ptr(lin[0]), _ptr(lin[1]), _ptr(lin[2])
+            a.lam_out0, a.lam_out1, a.lam_out2 = _ptr(lout[0]), _ptr(lout[1]), _ptr(lout[2])
+            a.rbar0, a.rbar1, a.rbar2 = _ptr(self._rbar[0]), _ptr(self._rbar[1]), _ptr(self._rbar[2])
+            a.n_bar, a.rate_bar = _ptr(self.n_bar), _ptr(self.rate_bar)
+            inflow = self._inflow_args(q) if self.inlet is not None else None
+            gauge = self._gauge_args(q[0], 0, lam0=lout[0], target=self._tgt) if G else None
+            calls = []
+            if inflow is not None:
+                calls.append((lib.gsw_flat_inflow_apply, (C.byref(inflow), s)))
+            calls.append((lib.gsw_adj_flat_step, (C.byref(a), s)))
+            if inflow is not None:
+                calls.append((lib.gsw_adj_flat_inflow, (C.byref(inflow), _ptr(lout[0]), _ptr(lout[1]), _ptr(lout[2]),
+                                                        _ptr(self.q_bar), s)))
+            if gauge is not None:
+                calls.append((lib.gsw_gauge_adjoint, (C.byref(gauge), s)))
+            return a, inflow, gauge, calls
+
+        def reverse_step(n, k, _keep=(p2, rows)):
+            lin, lout = self._lam[1], self._lam[0]
+            key = (k, lin is first)
+            if key not in made:
+                made[key] = build(k, lin, lout)
+            a, inflow, gauge, calls = made[key]
+            st = row0 + 128 * n
+            a.f.state, a.f.lam_target = st, st + lam_off
+            if inflow is not None:
+                inflow.state = st
+            if gauge is not None:
+                gauge.state = st
+            if lib.gsw_dt_finalize(C.byref(p2), C.c_void_p(st), s) != L.OK:
+                raise L.GswError("gsw_dt_finalize", -1, lib.gsw_last_error().decode(errors="replace"))
+            for fn, args in calls:
+                if fn(*args) != L.OK:
+                    raise L.GswError(fn.__name__, -1, lib.gsw_last_error().decode(errors="replace"))
+            self.kernel_launches += n_launch
+            self._lam = [lin, lout]
+
+        first = self._lam[1]
+        return reverse_step
 
     def adjoint_state(self, c=0):
         """Field c of the adjoint of the initial state after gradients() (slot-indexed)."""
