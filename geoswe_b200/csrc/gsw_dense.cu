@@ -43,72 +43,42 @@ __device__ __forceinline__ int bc_src(int kind, int g, int n, int ngh) {
     return kind == GSW_BC_WALL ? (n - ngh - 1 - k) : kind == GSW_BC_PERIODIC ? (ngh + k) : (n - ngh - 1);
 }
 
+// blockIdx.y is the ghost row (over every column, corners included) or, from 2 ngh on, the ghost
+// column (over the interior rows), so no thread divides a cell index: a step of a small grid
+// waits for this kernel.
 template <typename T>
 __global__ void bc_fill_kernel(T* q0, T* q1, T* q2, int nxp, int nyp, int ngh, int64_t pitch,
                                int kxm, int kxp, int kym, int kyp, const GswLoopState* st) {
     chain_begin();
     if (st != nullptr && st->done) return;
-    const int nyi = nyp - 2 * ngh, nxi = nxp - 2 * ngh;
-    const int64_t nX = (int64_t)2 * ngh * nyi;      // x-ghost cells at interior columns
-    const int64_t nY = (int64_t)2 * ngh * nxi;      // y-ghost cells at interior rows
-    const int64_t nC = (int64_t)4 * ngh * ngh;      // corners
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nX + nY + nC;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        int gi, gj, kx = GSW_BC_NONE, ky = GSW_BC_NONE;
-        if (t < nX) {
-            const int side = (int)(t / ((int64_t)ngh * nyi));
-            const int64_t rem = t - (int64_t)side * ngh * nyi;
-            const int k = (int)(rem / nyi);
-            gj = ngh + (int)(rem - (int64_t)k * nyi);
-            gi = side == 0 ? k : nxp - ngh + k;
-            kx = side == 0 ? kxm : kxp;
-        } else if (t < nX + nY) {
-            const int64_t u = t - nX;
-            const int side = (int)(u / ((int64_t)ngh * nxi));
-            const int64_t rem = u - (int64_t)side * ngh * nxi;
-            const int k = (int)(rem / nxi);
-            gi = ngh + (int)(rem - (int64_t)k * nxi);
-            gj = side == 0 ? k : nyp - ngh + k;
-            ky = side == 0 ? kym : kyp;
-            if (ky == GSW_BC_NONE) continue;
-        } else {
-            const int64_t u = t - nX - nY;
-            const int c = (int)(u / ((int64_t)ngh * ngh));
-            const int rem = (int)(u - (int64_t)c * ngh * ngh);
-            const int a = rem / ngh, bb = rem - a * ngh;
-            gi = (c & 1) ? nxp - ngh + a : a;
-            gj = (c & 2) ? nyp - ngh + bb : bb;
-            kx = (c & 1) ? kxp : kxm;
-            ky = (c & 2) ? kyp : kym;
-            if (ky == GSW_BC_NONE && kx == GSW_BC_NONE) continue;
-        }
-        const int64_t go = (int64_t)gi * pitch + gj;
+    const bool rows = (int)blockIdx.y < 2 * ngh;
+    const int layer = rows ? blockIdx.y : blockIdx.y - 2 * ngh;
+    const bool low = layer < ngh;
+    const int ghost = low ? layer : (rows ? nxp : nyp) - 2 * ngh + layer;
+    const int lo = rows ? 0 : ngh, hi = rows ? nyp : nxp - ngh;
+    for (int along = lo + blockIdx.x * blockDim.x + threadIdx.x; along < hi; along += gridDim.x * blockDim.x) {
+        const int gi = rows ? ghost : along, gj = rows ? along : ghost;
+        const int kx = !rows ? GSW_BC_NONE : low ? kxm : kxp;
+        const bool corner = rows && (gj < ngh || gj >= nyp - ngh);
+        const int ky = rows && !corner ? GSW_BC_NONE : gj < ngh ? kym : kyp;
+        if (kx == GSW_BC_NONE && ky == GSW_BC_NONE) continue;
         // value of the x pass at (row gi, column cj)
         auto xval = [&](int cj, T& a, T& u, T& v) {
-            if (kx == GSW_BC_NONE) { const int64_t o = (int64_t)gi * pitch + cj; a = q0[o]; u = q1[o]; v = q2[o]; return; }
             if (kx == GSW_BC_FALL) { a = (T)0; u = (T)0; v = (T)0; return; }
-            const int64_t o = (int64_t)bc_src(kx, gi, nxp, ngh) * pitch + cj;
+            const int64_t o = (int64_t)(kx == GSW_BC_NONE ? gi : bc_src(kx, gi, nxp, ngh)) * pitch + cj;
             a = q0[o]; u = q1[o]; v = q2[o];
             if (kx == GSW_BC_WALL) u = -u;
         };
         T a, u, v;
-        if (t < nX) {
-            xval(gj, a, u, v);
-            if (kx == GSW_BC_NONE) continue;
-        } else if (ky == GSW_BC_NONE) {            // corner left to the x pass
+        if (ky == GSW_BC_NONE) {                   // a ghost row, or a corner left to the x pass
             xval(gj, a, u, v);
         } else if (ky == GSW_BC_FALL) {
             a = (T)0; u = (T)0; v = (T)0;
         } else {
-            const int sj = bc_src(ky, gj, nyp, ngh);
-            if (t < nX + nY) {
-                const int64_t o = (int64_t)gi * pitch + sj;
-                a = q0[o]; u = q1[o]; v = q2[o];
-            } else {
-                xval(sj, a, u, v);
-            }
+            xval(bc_src(ky, gj, nyp, ngh), a, u, v);
             if (ky == GSW_BC_WALL) v = -v;
         }
+        const int64_t go = (int64_t)gi * pitch + gj;
         q0[go] = a; q1[go] = u; q2[go] = v;
     }
 }
@@ -238,16 +208,15 @@ extern "C" int gsw_bc_fill(const GswBcArgs* a, void* stream) {
         return set_error(GSW_ERR_INVALID, "bc: bad extents");
     for (int f = 0; f < 4; ++f)
         if (a->kinds[f] < 0 || a->kinds[f] > GSW_BC_NONE) return set_error(GSW_ERR_INVALID, "bc: bad kind %d", a->kinds[f]);
-    const int64_t n = (int64_t)2 * a->ngh * (a->nyp - 2 * a->ngh) + (int64_t)2 * a->ngh * (a->nxp - 2 * a->ngh) +
-                      (int64_t)4 * a->ngh * a->ngh;
-    const int grid = (int)std::min<int64_t>(sm_count() * 4, (n + 255) / 256);
+    if (a->ngh > 16383) return set_error(GSW_ERR_INVALID, "bc: ngh is too large");
+    const dim3 grid((unsigned)std::min((std::max(a->nxp, a->nyp) + 255) / 256, 64), (unsigned)(4 * a->ngh));
     cudaStream_t s = (cudaStream_t)stream;
     if (a->dtype == GSW_F32)
-        launch_chained(bc_fill_kernel<float>, dim3(grid), dim3(256), s, (float*)a->q0, (float*)a->q1, (float*)a->q2, a->nxp, a->nyp,
+        launch_chained(bc_fill_kernel<float>, grid, dim3(256), s, (float*)a->q0, (float*)a->q1, (float*)a->q2, a->nxp, a->nyp,
                                                    a->ngh, a->pitch, a->kinds[0], a->kinds[1], a->kinds[2],
                                                    a->kinds[3], a->state);
     else if (a->dtype == GSW_F64)
-        launch_chained(bc_fill_kernel<double>, dim3(grid), dim3(256), s, (double*)a->q0, (double*)a->q1, (double*)a->q2, a->nxp, a->nyp,
+        launch_chained(bc_fill_kernel<double>, grid, dim3(256), s, (double*)a->q0, (double*)a->q1, (double*)a->q2, a->nxp, a->nyp,
                                                     a->ngh, a->pitch, a->kinds[0], a->kinds[1], a->kinds[2],
                                                     a->kinds[3], a->state);
     else return set_error(GSW_ERR_INVALID, "bc: bad dtype");

@@ -98,9 +98,11 @@ template <> __device__ __forceinline__ float  dt_of<float>(const GswLoopState* s
 template <> __device__ __forceinline__ double dt_of<double>(const GswLoopState* st) { return st->dt; }
 
 // Binary64, and binary32 on rows too long for dense_rows_kernel's 32-bit offsets. STEP = false:
-// residual into o0..o2. STEP = true: updated state into o0..o2. REFPOW: as DenseRow's.
+// residual into o0..o2. STEP = true: updated state into o0..o2. REFPOW: as DenseRow's. Bound by
+// the binary64 operators' latency: 128 registers (139 without the cap) leave room for 16
+// warps per SM instead of 12, and the wave speed needs no block barrier (733x1021: 98 -> 89 us).
 template <typename T, bool STEP, bool REFPOW>
-__global__ void __launch_bounds__(256, 1) dense_march_kernel(DenseK<T> p) {
+__global__ void __maxnreg__(128) dense_march_kernel(DenseK<T> p) {
     chain_begin();
     if (STEP && p.st->done) return;                       // grid-uniform
     const int lane = threadIdx.x;
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(256, 1) dense_march_kernel(DenseK<T> p) {
             b_next = b_p2;
         }
     }
-    if (STEP && p.lam != nullptr) block_max_to(lam_local, p.lam);
+    if (STEP && p.lam != nullptr) warp_max_to(lam_local, p.lam);
 }
 
 // ------------------------------------------------------------------- binary32 (march_rows)
@@ -386,11 +388,12 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
         k.tile_rows = 4;
         for (int tr = 32; tr > 4; tr >>= 1)
             if (strips * ((nrows + tr - 1) / tr) >= want) { k.tile_rows = tr; break; }
-        // grids under four rows per resident warp: the shortest march that one wave of warps
-        // covers, since a step is then one march long (us per step, tile 4 against the rule's:
-        // 96^2 19.3 and 13.0 with one row, 256^2 19.3 and 14.8 with one, 512^2 24.5 and 23.7 with three)
-        if (sizeof(T) == 4 && strips * nrows < 4LL * sm_count() * 24)
-            k.tile_rows = (int)std::max<int64_t>(1, (strips * nrows + sm_count() * 24 - 1) / (sm_count() * 24));
+        // grids under four rows per resident warp (24 per SM at 80 registers, 16 in binary64): the
+        // shortest march that one wave of warps covers, since a step is then one march long (us per
+        // step, tile 4 and the rule's: 96^2 19.3 and 13.0 with one row, 256^2 19.3 and 14.8 with one,
+        // 512^2 24.5 and 23.7 with three; binary64 200^2 30.0 and 17.6 with one)
+        const int64_t wave = (int64_t)sm_count() * (sizeof(T) == 4 ? 24 : 16);
+        if (strips * nrows < 4 * wave) k.tile_rows = (int)std::max<int64_t>(1, (strips * nrows + wave - 1) / wave);
     }
     // dense_rows_kernel's offsets within a tile (rows -2 .. tile_rows + 1) are 32-bit
     const int64_t widest = std::max(k.pitch, std::max(k.cpitch, (int64_t)1));

@@ -138,3 +138,21 @@ def test_non_finite_state_is_reported():
             s.q[field, 20, 30] = float("nan")
             with pytest.raises(FloatingPointError):
                 s.run(1e9, max_steps=3)
+
+
+@pytest.mark.parametrize("nx,ny,ngh", [(5, 7, 2), (40, 300, 4), (2100, 2050, 2)])
+@pytest.mark.parametrize("kinds", [("wall", "fall"), ("periodic", "extrapolate")])
+def test_device_loop_equals_single_steps(nx, ny, ngh, kinds):
+    """Runs of one and of several steps against the host's single steps, ghost cells included,
+    on grids of a few cells and of several blocks per ghost row."""
+    from geoswe_b200 import Config, Mesh2D, Solver2D
+    q0, bed = extreme_state("film", nx, ny, seed=nx)
+    mesh = Mesh2D(nx=nx, ny=ny, dx=2.0, dy=2.0, ngh=ngh)
+    cfg = dict(bc_x=kinds[0], bc_y=kinds[1], friction="manning", manning_n=0.03)
+    s, o = (Solver2D(mesh, Config(**cfg), q0, bed, use_graphs=g) for g in (True, False))
+    for steps in (1, 3, 4):
+        assert s.run(1e9, max_steps=steps) == steps
+        for _ in range(steps):
+            o.step()
+        assert s.t == o.t and s.last_dt == o.last_dt
+        assert torch.equal(s.q, o.q)
