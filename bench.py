@@ -324,7 +324,7 @@ def run_gsw(args, rank, world):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": _traffic("dense", cells)[0],
                      "traffic_from": _traffic("dense", cells)[1],
-                     "kernel": "dense_march_kernel<float,true>", "kernel_ms": kern_ms,
+                     "kernel": "dense_rows_kernel<true>", "kernel_ms": kern_ms,
                      "bytes_per_cell": bpc, "peak_source": peak_kind},
         "issue": issue_roofline("dense", cells, kern_ms, m["clocks"]),
         "clocks": m["clocks"],
@@ -344,7 +344,7 @@ def run_gsw(args, rank, world):
             "value": cells * args.steps * world / (f["ms"] / 1e3), "unit": UNIT,
             "ms_per_step": f["ms"] / args.steps, "gpu_launches": int(f["launches"]),
             "roofline": {"bound": "hbm", "achieved": f_ach, "peak": peak, "unit": "GB/s", "frac": f_ach / peak,
-                         "kernel": "gsw_fast::dense_march_kernel<float,true>", "kernel_ms": f["kern_ms"],
+                         "kernel": "gsw_fast::dense_rows_kernel<true>", "kernel_ms": f["kern_ms"],
                          "peak_source": peak_kind},
             "issue": issue_roofline("dense_fast", cells, f["kern_ms"], f["clocks"]),
             "clocks": f["clocks"], "launch_shape": f["shape"]}
@@ -910,7 +910,7 @@ def run_tidal(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": _traffic("flat_tidal", cells)[0],
                          "traffic_from": _traffic("flat_tidal", cells)[1],
-                         "kernel": "flat_march_kernel<float,1>",
+                         "kernel": "flat_march_kernel<float,int,1>",
                          "kernel_ms": kern_ms, "bytes_per_cell": 38, "peak_source": peak_kind,
                          "brick_bytes_GBs": stored_bytes / (kern_ms / 1e3) / 1e9},
             "issue": issue_roofline("flat_tidal", cells, kern_ms, clocks) if args.arith == "exact" else None,

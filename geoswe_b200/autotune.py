@@ -45,7 +45,8 @@ def _key(kind, cells):
     except Exception:
         pass
     size = "small" if cells < 1 << 20 else ("medium" if cells < 1 << 24 else "large")
-    return f"{kind}|{dev}|{drv}|{size}"
+    # min_blocks names other register caps than in entries without the tag, which are not read
+    return f"{kind}|{dev}|{drv}|{size}|caps 80/96/64/72"
 
 
 def load(kind, cells):

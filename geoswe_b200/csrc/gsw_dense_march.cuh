@@ -9,7 +9,8 @@
 //     right lane with one warp shuffle;
 // so each face is evaluated once instead of twice, and no shared memory or block
 // barrier is needed on the step path. The new state's wave speed is reduced in
-// registers, then per block, then with one 64-bit atomicMax.
+// registers, then per warp, then with one 64-bit atomicMax. Binary32 takes the faces and
+// the march of gsw_face.cuh (dense_rows_kernel), binary64 the operators (dense_march_kernel).
 //
 // Included by gsw_dense.cu (exact arithmetic) and gsw_fast.cu (fast arithmetic, with
 // namespace gsw renamed), so each compilation has its own kernels.

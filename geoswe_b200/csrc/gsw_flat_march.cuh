@@ -4,8 +4,8 @@
 // One warp per brick of 30 x brick_h cells, the same column march as the dense kernel
 // (gsw_dense_march.cuh): lanes 1..30 are the brick's columns, lane 0 / lane 31 read the
 // edge columns of the left / right brick, and the two rows above and below come from
-// the bricks above and below. Every face is computed once from the shared core
-// (gsw_core.cuh), so active-cell residuals are bit-identical to the dense kernel's.
+// the bricks above and below. Every face is computed once by the code the dense kernel uses
+// (gsw_face.cuh; gsw_core.cuh in binary64), so active-cell residuals are bit-identical to its.
 //
 // Included by gsw_flat.cu (exact arithmetic) and gsw_fast.cu (fast arithmetic, with
 // namespace gsw renamed).
