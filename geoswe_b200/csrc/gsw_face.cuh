@@ -212,16 +212,26 @@ static __device__ __noinline__ void face_general(const FCell& L, const FCell& R,
     F.Fh = f.Fh; F.Fn = f.Fn; F.Ft = f.Ft; F.srcL = f.srcL; F.srcR = f.srcR;
 }
 
+// bad: whether a cell of the face is outside the ranges (a y-face: the cell to the left is; the
+// lane to the right holds the other).
 template <bool XAXIS>
 __device__ __forceinline__ void face(const FCell& L, const FCell& R, const FacePhys& p, bool bad, FFace& F) {
     const bool out = face_in<XAXIS>(L, R, p, F);
 #ifndef GSW_FAST_ARITH
-    if (__any_sync(0xffffffffu, bad || out)) {
-        const FCell a = L, b = R;              // copies: the march's own stay in registers
-        const FacePhys q = p;
-        FFace G;
-        face_general<XAXIS>(a, b, q, G);
-        F = G;
+    bool slow = bad || out;
+    if (__any_sync(0xffffffffu, slow)) {
+        if (!XAXIS) slow = __shfl_down_sync(0xffffffffu, bad, 1) || slow;      // the cell to the right
+        // a face of two cells below h_min is zero whatever their beds (no-data values among
+        // them), so it does not send its warp to the operators
+        if (__any_sync(0xffffffffu, slow && !(L.h < p.h_min && R.h < p.h_min))) {
+            const FCell a = L, b = R;          // copies: the march's own stay in registers
+            const FacePhys q = p;
+            FFace G;
+            face_general<XAXIS>(a, b, q, G);
+            F = G;
+        } else if (slow) {
+            F.Fh = F.Fn = F.Ft = F.srcL = F.srcR = 0.0f;
+        }
     }
 #endif
 }
@@ -335,7 +345,8 @@ __device__ __forceinline__ void march_rows(const A& acc, U& upd, int n, const Fa
         float rh, rhu, rhv;
         // the residual, in the reference's order per component (E, W, N, S): the leading
         // 0 - E + W is formed as W - E (the same rounding; only a zero's sign can differ)
-        if (__any_sync(0xffffffffu, bad_cur || bad_nx || !(cur.h < ph.h_min) || !(nx.h < ph.h_min))) {
+        // a row pair below h_min has no fluxes, whatever its beds
+        if (__any_sync(0xffffffffu, !(cur.h < ph.h_min) || !(nx.h < ph.h_min))) {
             FFace E;
             face<true>(cur, nx, ph, bad_cur || bad_nx, E);
             rh = wFh - E.Fh;
@@ -358,7 +369,7 @@ __device__ __forceinline__ void march_rows(const A& acc, U& upd, int n, const Fa
                 rhv = (((rhv - N.Fn) - N.srcL) + __shfl_up_sync(0xffffffffu, N.Fn, 1)) +
                       __shfl_up_sync(0xffffffffu, N.srcR, 1);
             }
-        } else {                               // every cell of the two rows below h_min: no fluxes
+        } else {                               // every cell of the two rows below h_min
             rh = wFh; rhu = wFn + wsR; rhv = wFt;
             wFh = wFn = wFt = wsR = 0.0f;
         }

@@ -1,0 +1,157 @@
+"""States and physics outside the ranges of the step kernels' faces (gsw_face.cuh): their values
+against the C oracle or another path, bit for bit, in the kernels of the production configuration
+(a class table on the dense mesh, the L2 wave speed on the compressed one, the ensemble, the
+adjoint), and what they cost, as a ratio of two times of the same kernels on one GPU.
+
+Each bound on a ratio lies between what the operators alone cost (at most 1.3 of the ordinary
+step) and what evaluating every row twice did (1.4 to 1.9).
+"""
+import ctypes as C
+import functools
+
+import numpy as np
+import pytest
+
+import oracle
+from tests._cases import pad_state, same
+from tests.test_face_gpu import KINDS, extreme_state
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+NTAB = np.array([0.02, 0.05, 0.09], np.float32)
+
+
+def _classes(nx, ny, seed):
+    return np.pad(np.random.default_rng(seed).integers(0, 3, (nx, ny)).astype(np.uint8), 2, mode="edge")
+
+
+def _solver(q0, bed, cls=True, **cfg):
+    from geoswe_b200 import Config, Mesh2D, Solver2D
+    nx, ny = bed.shape
+    kw = dict(bc_x="wall", bc_y="wall", friction="manning", arith="portable", h_min=1e-6)
+    kw.update(cfg)
+    s = Solver2D(Mesh2D(nx=nx, ny=ny, dx=2.0, dy=2.0, ngh=2), Config(**kw), q0, bed)
+    if cls:
+        s.set_manning_table(_classes(nx, ny, 1), NTAB)
+    return s
+
+
+def _oracle(q0, bed, **kw):
+    nx, ny = bed.shape
+    qp, bp = pad_state(q0, bed, 2, np.float32)
+    return oracle.OracleSolver2D(qp, bp, 2, 2.0, 2.0, kinds=["wall"] * 4, friction="manning",
+                                 ncls=_classes(nx, ny, 1), ntab=NTAB, **kw)
+
+
+def _same_runs(q0, bed, steps=4, **phys):
+    """Device-loop runs of the dense solver and the oracle."""
+    s, o = _solver(q0, bed, **phys), _oracle(q0, bed, **phys)
+    assert s.run(1e9, max_steps=steps) == o.run(1e9, max_steps=steps) == steps
+    assert s.t == o.t
+    assert same(s.q_interior.cpu().numpy(), o.q[:, 2:-2, 2:-2])
+
+
+# ---------------------------------------------------------------------------- no-data beds
+def _beds(value, seed=3, rim=True):
+    """A flowing state whose right half is dry, behind dry ground four cells wide or a ragged
+    shore, on beds of `value`."""
+    q0, bed = extreme_state("plain", 90, 128, seed=seed)
+    hit = np.zeros(bed.shape, bool)
+    hit[:, 70:] = True
+    if not rim:
+        hit |= np.random.default_rng(seed).random(bed.shape) < 0.05
+    q0[:, hit] = 0.0
+    if rim:
+        q0[:, :, 66:] = 0.0
+        bed[:, 66:] = 50.0
+    bed[hit] = value
+    return q0, bed
+
+
+@pytest.mark.parametrize("value", [99999.0, 1.0e6, -32768.0, 3.4e38])
+@pytest.mark.parametrize("rim", [True, False])
+def test_no_data_beds_match_oracle(value, rim):
+    if not rim and value > 1e30:
+        pytest.skip("water beside such a bed overflows")
+    _same_runs(*_beds(value, rim=rim))
+
+
+@pytest.mark.parametrize("arith", ["portable", "exact"])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_non_finite_beds_under_dry_ground(arith, value):
+    """Beds that the solver refuses and a caller of the C entry points may hold: two dry cells
+    exchange nothing whatever their beds, so the run is that of an ordinary high bed."""
+    q0, bed = _beds(50.0)
+    a, b = _solver(q0, bed, arith=arith), _solver(q0, bed, arith=arith)
+    b._b[:, 72:] = value
+    assert a.run(1e9, max_steps=6) == b.run(1e9, max_steps=6) == 6
+    assert a.t == b.t
+    assert torch.equal(a.q, b.q) and bool(torch.isfinite(b.q).all())
+    assert torch.equal(a.residual(), b.residual())
+
+
+# ----------------------------------------------------------------------------- what it costs
+@functools.lru_cache(maxsize=None)
+def _ground(nx=1536, ny=1500):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    z = torch.zeros((nx, ny), device="cuda")
+    n, amp = 4, 12.0
+    while n <= 1024:
+        c = torch.randn((1, 1, n, n), generator=g, device="cuda")
+        z += amp * torch.nn.functional.interpolate(c, (nx, ny), mode="bilinear", align_corners=True)[0, 0]
+        n, amp = 2 * n, amp / 2
+    z -= z.min()
+    level = z.reshape(-1)[::97].quantile(0.3)
+    film = 0.003 * torch.rand((nx, ny), generator=g, device="cuda")
+    h = torch.where(z < level, level - z, torch.where(film > 0.001, film, torch.zeros_like(film)))
+    u = 0.3 * torch.randn((2, nx, ny), generator=g, device="cuda")
+    cls = torch.randint(0, 3, (nx + 4, ny + 4), generator=g, device="cuda", dtype=torch.uint8)
+    return torch.stack([h, h * u[0], h * u[1]]), z, cls
+
+
+def _step_us(s, steps=16):
+    s.run(1e12, max_steps=steps)
+    best = 1e30
+    for _ in range(5):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record()
+        s.run(1e12, max_steps=steps)
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]))
+    return best * 1e3 / steps
+
+
+def _cost(flat=False, fs=None, change=None, **cfg):
+    from geoswe_b200.compressed import CompressedSolver
+    q, z, cls = _ground()
+    if change is not None:
+        q, z = change(q.clone(), z.clone())
+    s = _solver(q, z, cls=False, arith="exact", **dict(dict(bc_x="fall", bc_y="fall"), **cfg))
+    s.set_manning_table(cls, NTAB)
+    if flat:
+        m = np.zeros(tuple(z.shape), bool)
+        m[3:-3, 3:-3] = True
+        s.set_inside_mask(m)
+        s = CompressedSolver.from_dense(s, **(fs or {}))
+    return _step_us(s)
+
+
+def _costs_at_most(bound, changed, usual):
+    """Whether the time of `changed` is under `bound` of that of `usual`, in one of a few tries: the
+    host is shared and holds a launch up now and then."""
+    return any(_cost(**changed) < bound * _cost(**usual) for _ in range(4))
+
+
+def test_no_data_beds_cost_nothing_on_dry_rows():
+    def half(value):
+        def change(q, z):
+            q[:, :, 746:] = 0.0
+            z[:, 746:] = 60.0
+            z[:, 750:] = value
+            return q, z
+        return change
+    usual = dict(change=half(60.0))
+    assert _costs_at_most(1.15, dict(change=half(3.4e38)), usual)
+    assert _costs_at_most(1.15, dict(change=half(-3.4e38)), usual)
