@@ -80,6 +80,7 @@ __device__ __forceinline__ void load_state(const FlatMesh<T>& m, int64_t s, Cell
 // One row of kernel A in binary32: the update run backwards from the row's old depth and
 // residual, which march_rows recomputes as the forward step did.
 struct AdjTailRow {
+    static constexpr bool kDryZero = false;
     const AdjK<float>& p;
     double* s_nbar;
     int64_t base;                    // the lane's slot of row r0

@@ -249,6 +249,7 @@ struct DenseRows {
 // configuration takes the general kernel; both give the same bits.
 template <bool STEP, bool REFPOW, bool LEAN>
 struct DenseRow {
+    static constexpr bool kDryZero = kFastArith && !STEP;
     const DenseK<float>& p;
     int c, i0;
     bool out_lane;

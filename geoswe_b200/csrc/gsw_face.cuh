@@ -92,6 +92,12 @@ __host__ __device__ inline bool face_ranges(float g, float h_min, float h_cfl) {
     return g >= 1.0f && g <= 128.0f && h_min >= 0x1p-24f && h_min <= 1.0f && h_cfl >= 0x1p-24f && h_cfl <= 1.0f;
 }
 
+#ifdef GSW_FAST_ARITH
+constexpr bool kFastArith = true;
+#else
+constexpr bool kFastArith = false;
+#endif
+
 // A cell as its faces need it: hgx, hgy are half_d times the central bed gradients.
 struct FCell { float h, u, v, b, hgx, hgy; };
 
@@ -139,8 +145,11 @@ struct FacePhys { float inv_dx, inv_dy, hinv_dx, hinv_dy, half_dx, half_dy, g, g
 //     forced instead of the speeds;
 //   * the star flux is F + S (...) with S = min(SL, 0) on side L, max(SR, 0) on side R: S = 0
 //     exactly where the physical flux is meant, and its denominator is then set to 1;
-//   * a face whose two cells are below h_min gives zeros: its 1/d is set to zero.
-template <bool XAXIS>
+//   * a face whose two cells are below h_min gives zeros: its 1/d is set to zero. DRY_ZERO: also
+//     where their beds are not finite, which only the sources show, and only in the fast
+//     arithmetic (in the exact one such cells are flagged; 1.5 % of the fast step, which drops
+//     these cells' momenta in any case, so only the fast residual has it).
+template <bool XAXIS, bool DRY_ZERO>
 __device__ __forceinline__ bool face_in(const FCell& L, const FCell& R, const FacePhys& p, FFace& F) {
     const float z = 0.0f;
     const float zL = L.b + (XAXIS ? L.hgx : L.hgy), zR = R.b - (XAXIS ? R.hgx : R.hgy);
@@ -162,6 +171,10 @@ __device__ __forceinline__ bool face_in(const FCell& L, const FCell& R, const Fa
         const float kR = fmaxf(z, fminf(lowL ? INFINITY : -clip, wR));
         F.srcL = ((hg * (hL + L.h)) * ((zf0 - kL) - L.b)) * inv;
         F.srcR = ((hg * (hR + R.h)) * ((zf0 - kR) - R.b)) * inv;
+        if (DRY_ZERO) {
+            F.srcL = lowL && lowR ? z : F.srcL;
+            F.srcR = lowL && lowR ? z : F.srcR;
+        }
     }
     // HLLC
     const float aL = sqrt_in(p.g * hL), aR = sqrt_in(p.g * hR);
@@ -214,9 +227,9 @@ static __device__ __noinline__ void face_general(const FCell& L, const FCell& R,
 
 // bad: whether a cell of the face is outside the ranges (a y-face: the cell to the left is; the
 // lane to the right holds the other).
-template <bool XAXIS>
+template <bool XAXIS, bool DRY_ZERO>
 __device__ __forceinline__ void face(const FCell& L, const FCell& R, const FacePhys& p, bool bad, FFace& F) {
-    const bool out = face_in<XAXIS>(L, R, p, F);
+    const bool out = face_in<XAXIS, DRY_ZERO>(L, R, p, F);
 #ifndef GSW_FAST_ARITH
     bool slow = bad || out;
     if (__any_sync(0xffffffffu, slow)) {
@@ -307,7 +320,7 @@ __device__ __forceinline__ bool update_in(FState& s, bool friction, float n, flo
 //   A: the rows' data. state(k, h, hu, hv), bed(k); bed_out(k): of lane 0 (31) the bed left
 //      (right) of its own column.
 //   U: what is done with a row. pre(k): loads issued before the faces; row(k, h, rh, rhu, rhv):
-//      the row's old depth and residual.
+//      the row's old depth and residual. kDryZero: as face_in's DRY_ZERO.
 // The march starts one row early, for the x-face above row 0 alone. Rows -2 .. n + 1 are read.
 // `general` (warp-uniform): every row by the operators.
 constexpr int kMarchUnroll = 1;
@@ -348,7 +361,7 @@ __device__ __forceinline__ void march_rows(const A& acc, U& upd, int n, const Fa
         // a row pair below h_min has no fluxes, whatever its beds
         if (__any_sync(0xffffffffu, !(cur.h < ph.h_min) || !(nx.h < ph.h_min))) {
             FFace E;
-            face<true>(cur, nx, ph, bad_cur || bad_nx, E);
+            face<true, U::kDryZero>(cur, nx, ph, bad_cur || bad_nx, E);
             rh = wFh - E.Fh;
             rhu = (wFn - (E.Fn + E.srcL)) + wsR;
             rhv = wFt - E.Ft;
@@ -362,7 +375,7 @@ __device__ __forceinline__ void march_rows(const A& acc, U& upd, int n, const Fa
                 rn.hgy = __shfl_down_sync(0xffffffffu, cur.hgy, 1);
                 rn.hgx = rn.hgy;               // unused by a y-face
                 FFace N;
-                face<false>(cur, rn, ph, bad_cur, N);
+                face<false, U::kDryZero>(cur, rn, ph, bad_cur, N);
                 // the y-face left of the column comes from the lane to the left
                 rh = (rh - N.Fh) + __shfl_up_sync(0xffffffffu, N.Fh, 1);
                 rhu = (rhu - N.Ft) + __shfl_up_sync(0xffffffffu, N.Ft, 1);

@@ -154,6 +154,7 @@ __device__ __forceinline__ FlatRows<I> flat_rows(const FlatMesh<float>& m, const
 // general path.
 template <typename I, bool STEP, bool REFPOW, bool LEAN>
 struct FlatRow {
+    static constexpr bool kDryZero = kFastArith && !STEP;
     const FlatMesh<float>& m;
     const FlatPhys<float>& ph;
     I base;                          // the lane's slot of row 0

@@ -77,7 +77,7 @@ def test_no_data_beds_match_oracle(value, rim):
     _same_runs(*_beds(value, rim=rim))
 
 
-@pytest.mark.parametrize("arith", ["portable", "exact"])
+@pytest.mark.parametrize("arith", ["portable", "exact", "fast"])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 def test_non_finite_beds_under_dry_ground(arith, value):
     """Beds that the solver refuses and a caller of the C entry points may hold: two dry cells
