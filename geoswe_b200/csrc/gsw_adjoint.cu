@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128, MINB) adj_tail_kernel(AdjK<T> p) {
             const FlatRows<int64_t> acc = flat_rows<int64_t>(m, v, r0, lane);
             AdjTailRow upd = {p, s_nbar, bidx * v.BS + (int64_t)r0 * GSW_BRICK_PITCH + (lane - 1), m.bij[2 * bidx],
                               m.bij[2 * bidx + 1], r0, lane, dt, rate, frame, lane >= 1 && lane <= 30};
-            march_rows(acc, upd, r1 - r0, face_phys(ph), !face_ranges(ph.g, ph.h_min, ph.h_min));
+            march_rows(acc, upd, r1 - r0, face_phys(ph), !face_ranges(ph.g, ph.h_min));
             rate_acc = upd.rate_acc;
         }
     } else if (bidx < m.nb) {

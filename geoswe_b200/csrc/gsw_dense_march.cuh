@@ -41,7 +41,7 @@ struct DenseK {
     T h_cfl;
     int tile_rows;
     T g_recip;                   // RN(1/g) for the star depth's h / g, or 0 (gsw_core.cuh div_g)
-    bool general;                // binary32: outside face_ranges, every row by the operators
+    bool general;                // binary32: outside the ranges of gsw_face.cuh
     bool long_rows;              // binary32: rows too long for 32-bit offsets within a tile
 };
 
@@ -98,12 +98,13 @@ __device__ __forceinline__ T dt_of(const GswLoopState* st);
 template <> __device__ __forceinline__ float  dt_of<float>(const GswLoopState* st)  { return st->dt_f32; }
 template <> __device__ __forceinline__ double dt_of<double>(const GswLoopState* st) { return st->dt; }
 
-// Binary64, and binary32 on rows too long for dense_rows_kernel's 32-bit offsets. STEP = false:
-// residual into o0..o2. STEP = true: updated state into o0..o2. REFPOW: as DenseRow's. Bound by
-// the binary64 operators' latency: 128 registers (139 without the cap) leave room for 16
-// warps per SM instead of 12, and the wave speed needs no block barrier (733x1021: 98 -> 89 us).
-template <typename T, bool STEP, bool REFPOW>
-__global__ void __maxnreg__(128) dense_march_kernel(DenseK<T> p) {
+// The step by the operators: binary64, and binary32 outside the ranges of gsw_face.cuh or on rows
+// too long for dense_rows_kernel's 32-bit offsets. STEP = false: residual into o0..o2. STEP =
+// true: updated state into o0..o2. REFPOW, LEAN: as DenseRow's. Binary64 is bound by its operators'
+// latency: 128 registers (139 without the cap) leave room for 16 warps per SM instead of 12, and
+// the wave speed needs no block barrier (733x1021: 98 -> 89 us). Binary32 is bound by issue.
+template <typename T, bool STEP, int REGS, bool REFPOW, bool LEAN>
+__global__ void __maxnreg__(REGS) dense_march_kernel(DenseK<T> p) {
     chain_begin();
     if (STEP && p.st->done) return;                       // grid-uniform
     const int lane = threadIdx.x;
@@ -117,6 +118,7 @@ __global__ void __maxnreg__(128) dense_march_kernel(DenseK<T> p) {
     const int i0 = p.row_lo + blockIdx.y * p.tile_rows;
     const int i1 = min(i0 + p.tile_rows, p.row_hi);
     unsigned long long lam_local = 0ull;
+    uint32_t lam32 = 0u;        // binary32: the bits of the largest wave speed
 
     T dt = (T)0;
     T rate = (T)0;
@@ -152,6 +154,13 @@ __global__ void __maxnreg__(128) dense_march_kernel(DenseK<T> p) {
         cur = nx;
 
         for (int r = i0; r < i1; ++r) {
+            // loaded before the faces, as DenseRow::pre
+            uint8_t cls_r = 0;
+            T mh_r = (T)0;
+            if (LEAN && STEP && out_lane) {
+                cls_r = p.ncls[(int64_t)r * p.cpitch + c];
+                if (p.max_h != nullptr) mh_r = p.max_h[(int64_t)r * p.pitch + c];
+            }
             nx.h = pf_h; nx.hu = pf_hu; nx.hv = pf_hv;
             nx.b = b_next;
             const T b_p2 = pf_b;
@@ -188,7 +197,7 @@ __global__ void __maxnreg__(128) dense_march_kernel(DenseK<T> p) {
             }
 
             if (out_lane) {
-                const bool inside = (p.mask == nullptr) || (p.mask[(int64_t)r * p.mpitch + c] != 0);
+                const bool inside = LEAN || (p.mask == nullptr) || (p.mask[(int64_t)r * p.mpitch + c] != 0);
                 if (!inside) { rh = (T)0; rhu = (T)0; rhv = (T)0; }
                 const int64_t o = (int64_t)r * p.pitch + c;
                 if (!STEP) {
@@ -197,26 +206,31 @@ __global__ void __maxnreg__(128) dense_march_kernel(DenseK<T> p) {
                     T rr0 = rh;
                     if (inside) {
                         if (p.rain_kind == GSW_RAIN_UNIFORM) rr0 = rh + rate;
-                        else if (p.rain_kind == GSW_RAIN_GRIDDED)
+                        else if (!LEAN && p.rain_kind == GSW_RAIN_GRIDDED)
                             rr0 = rh + frame[(int64_t)(r - p.ngh) * (p.nyp - 2 * p.ngh) + (c - p.ngh)];
                     }
                     T h = cur.h + dt * rr0;
                     T hu = ldg_at(p.q1, p.pitch, r, c) + dt * rhu;     // reloaded: not carried down the march
                     T hv = ldg_at(p.q2, p.pitch, r, c) + dt * rhv;
                     T n = (T)0;
-                    if (p.friction_kind == GSW_FRICTION_TABLE)
+                    if (LEAN) n = p.ntab[cls_r];
+                    else if (p.friction_kind == GSW_FRICTION_TABLE)
                         n = p.ncls ? p.ntab[p.ncls[(int64_t)r * p.cpitch + c]] : p.ntab[0];
                     else if (p.friction_kind == GSW_FRICTION_FIELD) n = p.nfield[o];
-                    wetdry_friction<T>(h, hu, hv, p.friction_kind != GSW_FRICTION_NONE, n, dt, p.g,
-                                       p.h_min, p.vcap, p.quad != 0, p.keep_h != 0, REFPOW);
+                    wetdry_friction<T>(h, hu, hv, LEAN || p.friction_kind != GSW_FRICTION_NONE, n, dt, p.g,
+                                       p.h_min, p.vcap, LEAN || p.quad != 0, LEAN || p.keep_h != 0, REFPOW);
                     p.o0[o] = h; p.o1[o] = hu; p.o2[o] = hv;
-                    if (p.max_h != nullptr && h > p.max_h[o]) p.max_h[o] = h;
-                    if (p.lam != nullptr) {
-                        const bool skip = (p.cfl_skip != nullptr) &&
+                    if (p.max_h != nullptr && h > (LEAN ? mh_r : p.max_h[o])) p.max_h[o] = h;
+                    if (LEAN || p.lam != nullptr) {
+                        const bool skip = !LEAN && (p.cfl_skip != nullptr) &&
                             p.cfl_skip[(int64_t)(r - p.ngh) * (p.nyp - 2 * p.ngh) + (c - p.ngh)] != 0;
                         if (!skip) {
-                            const unsigned long long lb = lam_dense_bits(h, hu, hv, p.g, p.h_cfl);
-                            lam_local = lb > lam_local ? lb : lam_local;
+                            if constexpr (sizeof(T) == 4) {
+                                lam32 = max(lam32, lam_dense_bits32(h, hu, hv, p.g, p.h_cfl));
+                            } else {
+                                const unsigned long long lb = lam_dense_bits(h, hu, hv, p.g, p.h_cfl);
+                                lam_local = lb > lam_local ? lb : lam_local;
+                            }
                         }
                     }
                 }
@@ -225,7 +239,8 @@ __global__ void __maxnreg__(128) dense_march_kernel(DenseK<T> p) {
             b_next = b_p2;
         }
     }
-    if (STEP && p.lam != nullptr) warp_max_to(lam_local, p.lam);
+    if constexpr (sizeof(T) == 4) lam_local = lam_bits_of32(lam32);
+    if (STEP && (LEAN || p.lam != nullptr)) warp_max_to(lam_local, p.lam);
 }
 
 // ------------------------------------------------------------------- binary32 (march_rows)
@@ -294,7 +309,7 @@ struct DenseRow {
         s.hv = __ldg(p.q2 + base + o) + dt * rhv;
         const float n = LEAN ? p.ntab[cls] : manning(r, r * p.pitch + c);
         const bool fric = LEAN || p.friction_kind != GSW_FRICTION_NONE;
-        bool slow = p.general || (!LEAN && (p.quad == 0 || p.keep_h == 0));
+        bool slow = (kFastArith && p.general) || (!LEAN && (p.quad == 0 || p.keep_h == 0));
         if (!slow) slow = update_in<false, REFPOW>(s, fric, n, dt, p.g, p.h_min, p.vcap, p.h_cfl);
         if (slow) {
             FState g = s;                               // a copy: s itself stays in registers
@@ -336,7 +351,7 @@ __global__ void __maxnreg__(REGS) dense_rows_kernel(DenseK<float> p) {
                                lane == 0 ? max(c - 1, 0) : min(c + 1, p.nyp - 1)};
         const FacePhys ph = {p.inv_dx, p.inv_dy, 0.5f * p.inv_dx, 0.5f * p.inv_dy, p.half_dx, p.half_dy,
                              p.g, p.g_recip != 0.0f ? p.g_recip : rcp_in(p.g), p.h_min};
-        march_rows(acc, upd, n, ph, p.general);
+        march_rows(acc, upd, n, ph, false);
     }
     if (STEP && (LEAN || p.lam != nullptr)) warp_max_to(lam_bits_of32(upd.lam), p.lam);
 }
@@ -381,7 +396,8 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
     k.ntab = (const T*)a->n_tab; k.nfield = (const T*)a->n_field;
     k.vcap = (T)a->vcap; k.quad = a->quadratic; k.keep_h = a->keep_h;
     k.max_h = (T*)a->max_h; k.cfl_skip = a->cfl_skip; k.h_cfl = (T)a->h_cfl;
-    k.general = !face_ranges((float)k.g, (float)k.h_min, (float)k.h_cfl);
+    // the wave speed's floor only has to keep its root in the proven range (update_in)
+    k.general = !face_ranges((float)k.g, (float)k.h_min) || !((float)k.h_cfl >= 0x1p-90f);
     if (a->tile_rows > 0) {
         k.tile_rows = a->tile_rows;
     } else {   // rows per warp: the longest march (<= 32 rows) that still gives twice the resident warps
@@ -398,7 +414,7 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
         if (strips * nrows < 4 * wave) k.tile_rows = (int)std::max<int64_t>(1, (strips * nrows + wave - 1) / wave);
     }
     // dense_rows_kernel's offsets within a tile (rows -2 .. tile_rows + 1) are 32-bit
-    const int64_t widest = std::max(k.pitch, std::max(k.cpitch, (int64_t)1));
+    const int64_t widest = std::max(k.pitch, k.ncls ? k.cpitch : (int64_t)1);
     k.long_rows = INT32_MAX / widest < 5;
     if (!k.long_rows) k.tile_rows = (int)std::min<int64_t>(k.tile_rows, INT32_MAX / widest - 4);
     if (step) {
@@ -433,13 +449,16 @@ inline void launch_rows_caps(const DenseK<float>& k, int minb, dim3 grid, dim3 b
 
 template <bool STEP, bool REFPOW>
 inline void launch_shape(const DenseK<float>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
-    if (k.long_rows) launch_chained(dense_march_kernel<float, STEP, REFPOW>, grid, block, s, k);
-    else if (STEP && lean_config(k)) launch_rows_caps<STEP, REFPOW, STEP>(k, minb, grid, block, s);
+    const bool lean = STEP && lean_config(k);
+    if (k.long_rows || (!kFastArith && k.general)) {
+        if (lean) launch_chained(dense_march_kernel<float, STEP, 64, REFPOW, STEP>, grid, block, s, k);
+        else launch_chained(dense_march_kernel<float, STEP, 64, REFPOW, false>, grid, block, s, k);
+    } else if (lean) launch_rows_caps<STEP, REFPOW, STEP>(k, minb, grid, block, s);
     else launch_rows_caps<STEP, REFPOW, false>(k, minb, grid, block, s);
 }
 template <bool STEP, bool REFPOW>
 inline void launch_shape(const DenseK<double>& k, int, dim3 grid, dim3 block, cudaStream_t s) {
-    launch_chained(dense_march_kernel<double, STEP, false>, grid, block, s, k);
+    launch_chained(dense_march_kernel<double, STEP, 128, false, false>, grid, block, s, k);
 }
 
 template <typename T, bool STEP>

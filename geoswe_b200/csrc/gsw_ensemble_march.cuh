@@ -124,8 +124,8 @@ __global__ void __maxnreg__(REGS) ensemble_step_kernel(GswEnsembleArgs a, FlatMe
         const FlatPhys<float> ph = member_phys(mb, REFPOW ? 1 : 0);
         const float dt = st->dt_f32;
         const float rate = (mb.rain_kind == GSW_RAIN_UNIFORM) ? mb.rain[st->rain_idx] : 0.0f;
-        unsigned long long lam = flat_brick<float, I, true, REFPOW, LEAN>(m, ph, b, seg * m.bh / S, (seg + 1) * m.bh / S,
-                                                                  dt, rate, nullptr);
+        unsigned long long lam = flat_brick<float, I, true, REFPOW, LEAN, false>(
+            m, ph, b, seg * m.bh / S, (seg + 1) * m.bh / S, dt, rate, nullptr, !face_ranges(ph.g, ph.h_min));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long w = __shfl_xor_sync(0xffffffffu, lam, o);

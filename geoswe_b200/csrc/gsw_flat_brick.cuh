@@ -48,6 +48,7 @@ template <typename T>
 struct FlatK {
     FlatMesh<T> m; FlatPhys<T> ph; const GswLoopState* st; unsigned long long* lam; int segs;
     int64_t b0, b1;    // bricks [b0, b1) are stepped
+    bool general;      // binary32: outside the ranges of gsw_face.cuh
 };
 
 // Slot of brick-relative (row, lane). Lanes 0/31 of the rows above/below the brick are
@@ -203,7 +204,9 @@ struct FlatRow {
             s.hu = s.hu + dt * rhu;
             s.hv = s.hv + dt * rhv;
             const float n = m.ncls ? ph.ntab[LEAN ? cls : m.ncls[o]] : ph.ntab[0];
-            bool slow = general || (!LEAN && (ph.quad == 0 || ph.keep_h == 0));
+            // a wet cell whose wave speed divides by h_min_cfl instead of its depth
+            bool slow = general || (!LEAN && (ph.quad == 0 || ph.keep_h == 0)) ||
+                        (s.h < ph.h_min_cfl && !(s.h < ph.h_min));
             if (!slow) slow = update_in<true, REFPOW>(s, true, n, dt, ph.g, ph.h_min, ph.vcap, ph.h_min);
             if (slow) {
                 FState g = s;                         // a copy: s itself stays in registers
@@ -223,15 +226,16 @@ struct FlatRow {
     }
 };
 
-// Rows [r0, r1) of one brick in binary64 (the adjoint's derivative checks).
-template <bool STEP>
-__device__ __forceinline__ unsigned long long flat_brick_f64(const FlatMesh<double>& m, const FlatPhys<double>& ph,
-                                                             const BrickView& v, int bi, int bj, int r0, int r1,
-                                                             double dt, double rate, const double* frame) {
-    using T = double;
+// Rows [r0, r1) of one brick by the operators: binary64 (the adjoint's derivative checks), and
+// binary32 outside the ranges of gsw_face.cuh. Template parameters and result as flat_brick's.
+template <typename T, bool STEP, bool REFPOW, bool LEAN>
+__device__ __forceinline__ unsigned long long flat_brick_operators(const FlatMesh<T>& m, const FlatPhys<T>& ph,
+                                                                   const BrickView& v, int bi, int bj, int r0, int r1,
+                                                                   T dt, T rate, const T* frame) {
     const int lane = threadIdx.x;
     const int64_t bidx = v.self;
     unsigned long long lam_local = 0ull;
+    uint32_t lam32 = 0u;             // binary32: the L2 norm's key
     const int bh = m.bh;
     Cell<T> cur, nx;
     const T b_m2 = __ldg(m.b + v.slot(r0 - 2, lane));
@@ -252,6 +256,15 @@ __device__ __forceinline__ unsigned long long flat_brick_f64(const FlatMesh<doub
     srm_face<T, true>(cur, nx, ph.half_dx, ph.inv_dx, ph.g, ph.h_min, Wf, ph.g_recip);
     cur = nx;
     for (int r = r0; r < r1; ++r) {
+        // loaded before the faces, as FlatRow::pre
+        uint8_t f_r = 0, cls_r = 0;
+        T mh_r = (T)0;
+        if (LEAN && STEP && lane >= 1 && lane <= 30) {
+            const int64_t o = bidx * v.BS + (int64_t)r * GSW_BRICK_PITCH + (lane - 1);
+            f_r = m.flags[o];
+            if (m.ncls) cls_r = m.ncls[o];
+            if (m.max_h != nullptr) mh_r = m.max_h[o];
+        }
         nx.h = pf_h; nx.hu = pf_hu; nx.hv = pf_hv;
         nx.b = b_next;
         const T b_p2 = pf_b;
@@ -286,7 +299,7 @@ __device__ __forceinline__ unsigned long long flat_brick_f64(const FlatMesh<doub
         }
         if (lane >= 1 && lane <= 30) {
             const int64_t o = bidx * v.BS + (int64_t)r * GSW_BRICK_PITCH + (lane - 1);
-            const uint8_t f = m.flags[o];
+            const uint8_t f = (LEAN && STEP) ? f_r : m.flags[o];
             if (f & GSW_SLOT_STORED) {
                 const bool active = (f & GSW_SLOT_ACTIVE) != 0;
                 if (!STEP) {
@@ -294,43 +307,52 @@ __device__ __forceinline__ unsigned long long flat_brick_f64(const FlatMesh<doub
                     m.o0[o] = rh; m.o1[o] = rhu; m.o2[o] = rhv;
                 } else if (!active) {
                     m.o0[o] = cur.h; m.o1[o] = __ldg(m.q1 + o); m.o2[o] = __ldg(m.q2 + o);
-                    if (m.max_h != nullptr && cur.h > m.max_h[o]) m.max_h[o] = cur.h;
+                    if (m.max_h != nullptr && cur.h > (LEAN ? mh_r : m.max_h[o])) m.max_h[o] = cur.h;
                 } else {
                     T rr0 = rh;
                     if (ph.rain_kind == GSW_RAIN_UNIFORM) rr0 = rr0 + rate;
-                    else if (ph.rain_kind == GSW_RAIN_GRIDDED) {
+                    else if (!LEAN && ph.rain_kind == GSW_RAIN_GRIDDED) {
                         const int i = bi * bh + r, j = bj * GSW_BRICK_W + (lane - 1);
                         rr0 = rr0 + frame[(int64_t)(i - ph.ngh) * ph.ny + (j - ph.ngh)];
-                    } else if (ph.rain_kind == GSW_RAIN_LOOKUP) {
+                    } else if (!LEAN && ph.rain_kind == GSW_RAIN_LOOKUP) {
                         rr0 = rr0 + frame[ph.lookup[o]];
                     }
                     T h = cur.h + dt * rr0;
                     T hu = __ldg(m.q1 + o) + dt * rhu;       // reloaded: not carried down the march
                     T hv = __ldg(m.q2 + o) + dt * rhv;
-                    const T n = m.ncls ? ph.ntab[m.ncls[o]] : ph.ntab[0];
+                    const T n = m.ncls ? ph.ntab[LEAN ? cls_r : m.ncls[o]] : ph.ntab[0];
                     wetdry_friction<T>(h, hu, hv, true, n, dt, ph.g, ph.h_min, ph.vcap,
-                                       ph.quad != 0, ph.keep_h != 0, false);
+                                       LEAN || ph.quad != 0, LEAN || ph.keep_h != 0, REFPOW);
                     m.o0[o] = h; m.o1[o] = hu; m.o2[o] = hv;
-                    if (m.max_h != nullptr && h > m.max_h[o]) m.max_h[o] = h;
-                    const unsigned long long lb = lam_flat_bits(h, hu, hv, ph.g, ph.h_min, ph.h_min_cfl, ph.linf != 0);
-                    lam_local = lb > lam_local ? lb : lam_local;
+                    if (m.max_h != nullptr && h > (LEAN ? mh_r : m.max_h[o])) m.max_h[o] = h;
+                    if (sizeof(T) == 4 && (LEAN || ph.linf == 0)) {
+                        lam32 = max(lam32, lam_flat_bits32((float)h, (float)hu, (float)hv, (float)ph.g, (float)ph.h_min,
+                                                           (float)ph.h_min_cfl));
+                    } else {
+                        const unsigned long long lb = lam_flat_bits(h, hu, hv, ph.g, ph.h_min, ph.h_min_cfl, ph.linf != 0);
+                        lam_local = lb > lam_local ? lb : lam_local;
+                    }
                 }
             }
         }
         cur = nx;
         b_next = b_p2;
     }
-    return lam_local;
+    const unsigned long long l = lam_bits_of32(lam32);
+    return l > lam_local ? l : lam_local;
 }
 
 // Rows [r0, r1) of one brick, walked by one warp. A segment reads rows r0-2 .. r1+1 through
 // the brick view (the bricks above and below past the brick's edge) and recomputes the x-face
 // above row r0 from the same inputs as the face below row r0-1, so splitting a brick's rows
 // among warps changes no value. STEP: the fused step (returns this lane's wave speed bits);
-// otherwise the residual. `frame` is the gridded rain frame, or null. I: as FlatRows.
-template <typename T, typename I, bool STEP, bool REFPOW, bool LEAN>
+// otherwise the residual. `frame` is the gridded rain frame, or null. I: as FlatRows. OPERATORS:
+// every row by the operators; general (warp-uniform): the same where it is known on the device only
+// (an ensemble's member), by the rows' fallback.
+template <typename T, typename I, bool STEP, bool REFPOW, bool LEAN, bool OPERATORS>
 __device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, const FlatPhys<T>& ph, int64_t bidx,
-                                                         int r0, int r1, T dt, T rate, const T* frame) {
+                                                         int r0, int r1, T dt, T rate, const T* frame,
+                                                         bool general) {
     const int lane = threadIdx.x;
     BrickView v;
     v.BS = (int64_t)m.bh * GSW_BRICK_PITCH;
@@ -340,16 +362,15 @@ __device__ __forceinline__ unsigned long long flat_brick(const FlatMesh<T>& m, c
     v.left = m.bnbr[4 * bidx + 2]; v.right = m.bnbr[4 * bidx + 3];
     v.zero = m.nb;
     const int bi = m.bij[2 * bidx], bj = m.bij[2 * bidx + 1];
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (sizeof(T) == 4 && !OPERATORS) {
         const FlatRows<I> acc = flat_rows<I>(m, v, r0, lane);
-        const bool general = !face_ranges(ph.g, ph.h_min, ph.h_min_cfl) || ph.h_min_cfl != ph.h_min;
         FlatRow<I, STEP, REFPOW, LEAN> upd = {m, ph, (I)(bidx * v.BS) + (lane - 1), bi, bj, r0, lane, dt, rate, frame, general,
                                            lane >= 1 && lane <= 30};
         march_rows(acc, upd, r1 - r0, face_phys(ph), general);
         const unsigned long long l = lam_bits_of32(upd.lam32);
         return LEAN || l > upd.lam64 ? l : upd.lam64;
     } else {
-        return flat_brick_f64<STEP>(m, ph, v, bi, bj, r0, r1, dt, rate, frame);
+        return flat_brick_operators<T, STEP, REFPOW, LEAN>(m, ph, v, bi, bj, r0, r1, dt, rate, frame);
     }
 }
 

@@ -14,7 +14,7 @@
 
 namespace gsw {
 
-template <typename T, typename I, bool STEP, int REGS, bool REFPOW, bool LEAN>
+template <typename T, typename I, bool STEP, int REGS, bool REFPOW, bool LEAN, bool OPERATORS>
 __global__ void __maxnreg__(REGS) flat_march_kernel(FlatK<T> p) {
     chain_begin();
     if (STEP && p.st->done) return;
@@ -32,8 +32,9 @@ __global__ void __maxnreg__(REGS) flat_march_kernel(FlatK<T> p) {
         if (p.ph.rain_kind == GSW_RAIN_LOOKUP) frame = p.ph.rain + (int64_t)p.st->rain_idx * p.ph.ncol;
     }
     if (bidx < p.b1)
-        lam_local = flat_brick<T, I, STEP, REFPOW, LEAN>(p.m, p.ph, bidx, seg * p.m.bh / p.segs,
-                                                         (seg + 1) * p.m.bh / p.segs, dt, rate, frame);
+        lam_local = flat_brick<T, I, STEP, REFPOW, LEAN, OPERATORS>(p.m, p.ph, bidx, seg * p.m.bh / p.segs,
+                                                                    (seg + 1) * p.m.bh / p.segs, dt, rate, frame,
+                                                                    kFastArith && p.general);
     if (STEP && p.lam != nullptr) warp_max_to(lam_local, p.lam);
 }
 
@@ -59,6 +60,7 @@ inline int fill_flat(const GswFlatArgs* a, FlatK<T>& k, bool step) {
     ph.lookup = a->rain_lookup; ph.ncol = a->rain_ncol;
     ph.g_recip = sizeof(T) == 4 ? (T)div_const_recip((float)a->g) : (T)0;
     ph.ref_pow = a->arith == GSW_ARITH_EXACT ? 1 : 0;
+    k.general = !face_ranges((float)ph.g, (float)ph.h_min);
     k.st = a->state; k.lam = (unsigned long long*)a->lam_target;
     k.segs = a->segments > 0 ? a->segments : auto_segments(a->n_bricks, (int64_t)sm_count() * 24, a->brick_h);
     if (k.segs != 1 && k.segs != 2 && k.segs != 4) return set_error(GSW_ERR_INVALID, "flat: segments must be 0, 1, 2 or 4");
@@ -86,10 +88,10 @@ inline int fill_flat(const GswFlatArgs* a, FlatK<T>& k, bool step) {
 template <bool STEP, bool REFPOW, bool LEAN>
 inline void launch_flat_caps(const FlatK<float>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
     const dim3 b(32, W);
-    if (STEP && mb == 3) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 96 : 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
-    else if (STEP && mb == 4) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 64 : 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
-    else if (STEP && mb == 5) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 72 : 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
-    else launch_chained(flat_march_kernel<float, int, STEP, 80, REFPOW, LEAN>, dim3(blocks), b, s, k);
+    if (STEP && mb == 3) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 96 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
+    else if (STEP && mb == 4) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 64 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
+    else if (STEP && mb == 5) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 72 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
+    else launch_chained(flat_march_kernel<float, int, STEP, 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
 }
 
 // The production configuration (the LEAN kernel: rain none or uniform, quadratic
@@ -98,14 +100,19 @@ template <bool STEP, bool REFPOW>
 inline void launch_flat_shape(const FlatK<float>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
     const bool lean = k.ph.rain_kind != GSW_RAIN_GRIDDED && k.ph.rain_kind != GSW_RAIN_LOOKUP &&
                       k.ph.quad != 0 && k.ph.keep_h != 0 && k.ph.linf == 0;
-    if ((k.m.nb + 1) * (int64_t)k.m.bh * GSW_BRICK_PITCH > INT32_MAX)
-        launch_chained(flat_march_kernel<float, int64_t, STEP, 128, REFPOW, false>, dim3(blocks), dim3(32, W), s, k);
+    if (!kFastArith && k.general) {
+        if (STEP && lean)
+            launch_chained(flat_march_kernel<float, int64_t, STEP, 64, REFPOW, STEP, true>, dim3(blocks), dim3(32, W), s, k);
+        else
+            launch_chained(flat_march_kernel<float, int64_t, STEP, 64, REFPOW, false, true>, dim3(blocks), dim3(32, W), s, k);
+    } else if ((k.m.nb + 1) * (int64_t)k.m.bh * GSW_BRICK_PITCH > INT32_MAX)
+        launch_chained(flat_march_kernel<float, int64_t, STEP, 128, REFPOW, false, false>, dim3(blocks), dim3(32, W), s, k);
     else if (STEP && lean) launch_flat_caps<STEP, REFPOW, STEP>(k, mb, blocks, W, s);
     else launch_flat_caps<STEP, REFPOW, false>(k, mb, blocks, W, s);
 }
 template <bool STEP, bool REFPOW>
 inline void launch_flat_shape(const FlatK<double>& k, int, unsigned blocks, int W, cudaStream_t s) {
-    launch_chained(flat_march_kernel<double, int64_t, STEP, 200, false, false>, dim3(blocks), dim3(32, W), s, k);
+    launch_chained(flat_march_kernel<double, int64_t, STEP, 200, false, false, true>, dim3(blocks), dim3(32, W), s, k);
 }
 
 template <typename T, bool STEP>

@@ -52,6 +52,48 @@ def _same_runs(q0, bed, steps=4, **phys):
     assert same(s.q_interior.cpu().numpy(), o.q[:, 2:-2, 2:-2])
 
 
+# ------------------------------------------------------------------- the production kernels
+def _compressed(q0, bed, fs=None, **cfg):
+    from geoswe_b200.compressed import CompressedSolver
+    nx, ny = bed.shape
+    s = _solver(q0, bed, bc_x="fall", bc_y="fall", **cfg)
+    mask = np.zeros((nx, ny), bool)
+    mask[3:-3, 3:-3] = True
+    mask[20:30, 20:40] = False
+    s.set_inside_mask(mask)
+    return CompressedSolver.from_dense(s, **(fs or {}))
+
+
+def _flat_oracle(cs):
+    q = [cs.flat(c).cpu().numpy() for c in range(3)]
+    o = oracle.OracleFlat(cs.nbr, cs.is_active, q, cs._b[cs._slot].cpu().numpy(), cs.dx, g=cs.g,
+                          ncls=cs._ncls[cs._slot].cpu().numpy(), ntab=NTAB, linf=cs.cfl_linf)
+    o.h_min, o.h_min_cfl = cs.h_min, cs.h_min_cfl
+    return o
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("fs", [{}, dict(g=981.0), dict(h_min=1e-8), dict(h_min=1e-7)],
+                         ids=["earth", "g981", "h_min1e-8", "h_min1e-7"])
+def test_extreme_states_on_the_compressed_mesh_with_the_l2_speed(kind, fs):
+    """h_min 1e-7 leaves films under the wave speed's floor h_min_cfl (1e-6)."""
+    q0, bed = extreme_state(kind, 61, 67, seed=9)
+    cs = _compressed(q0, bed, fs)
+    o = _flat_oracle(cs)
+    assert cs.run(1e9, max_steps=4) == o.run(1e9, max_steps=4) == 4
+    assert cs.t == o.t
+    for c in range(3):
+        assert same(cs.flat(c).cpu().numpy(), o.q[c]), c
+
+
+@pytest.mark.parametrize("h_min_cfl", [1e-3, 2.0])
+def test_wave_speed_floor_of_the_dense_step(h_min_cfl):
+    q0, bed = extreme_state("film", 61, 64, seed=2)
+    s, o = _solver(q0, bed, h_min_cfl=h_min_cfl), _oracle(q0, bed, h_cfl=h_min_cfl)
+    assert s.run(1e9, max_steps=4) == o.run(1e9, max_steps=4)
+    assert s.t == o.t and same(s.q_interior.cpu().numpy(), o.q[:, 2:-2, 2:-2])
+
+
 # ---------------------------------------------------------------------------- no-data beds
 def _beds(value, seed=3, rim=True):
     """A flowing state whose right half is dry, behind dry ground four cells wide or a ragged
@@ -155,3 +197,13 @@ def test_no_data_beds_cost_nothing_on_dry_rows():
     usual = dict(change=half(60.0))
     assert _costs_at_most(1.15, dict(change=half(3.4e38)), usual)
     assert _costs_at_most(1.15, dict(change=half(-3.4e38)), usual)
+
+
+@pytest.mark.parametrize("cfg", [dict(g=981.0), dict(h_min=1e-8), dict(h_min_cfl=2.0)])
+def test_physics_outside_the_ranges_costs_the_operators(cfg):
+    assert _costs_at_most(1.5, cfg, {})
+
+
+@pytest.mark.parametrize("fs,bound", [(dict(g=981.0), 1.6), (dict(h_min=1e-8), 1.6), (dict(h_min=1e-7), 1.2)])
+def test_compressed_physics_outside_the_ranges_costs_the_operators(fs, bound):
+    assert _costs_at_most(bound, dict(flat=True, fs=fs), dict(flat=True))
