@@ -18,7 +18,7 @@
 //     a 2^s - b M = c for an odd M and |c| <= 2; all such pairs (|c| <= 8) are enumerated by
 //     the test and round correctly. Quotients by one divisor share y.
 // The two hold while nothing underflows, so operands outside stated ranges (a non-finite
-// value, a depth, bed or speed above 2^14, ...) raise a flag, and the row's face or update is
+// value, a depth, bed or speed above 2^17, ...) raise a flag, and the row's face or update is
 // evaluated again by the operators (srm_face, wetdry_friction): every value equals the IEEE
 // operators' in either case. A nonzero momentum under 2^-100, which a long run holds in up to a
 // cell in a hundred (friction and upwinding shrink it until it stays at a few binary32
@@ -84,7 +84,14 @@ __device__ __forceinline__ float div_in(float a, float b, float y) {
 __device__ __forceinline__ uint32_t low_key(float x) { return 2u * __float_as_uint(x) - 1u; }
 __device__ __forceinline__ uint32_t min3(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u32(a, b, c); }
 #define GSW_KEY(e) (2u * ((uint32_t)(127 + (e)) << 23) - 1u)       // low_key(2^e)
-constexpr float kFaceMax = 0x1p14f;    // depths, beds and speeds above this are left to the operators
+// Depths, beds and speeds above this are left to the operators. With it as the limit M of a
+// cell's |h| + |b| + |u| + |v|, a face's depths are at most 4 M, its wave speeds under 4 M (under 8 M
+// from a velocity), the star speed's denominator under 2^6 M^2 = 2^40 and its numerator under
+// 2^8 M^3 = 2^59, so that every quotient of a numerator above 2^-80 is a normal number and its
+// residual exact. 2^17 leaves the usual no-data values (-9999,
+// -32768, 99999) and elevations in feet or centimetres to these faces: at 2^14, terrain lifted by
+// 20000 took 145 us per step where 81 is enough (1536x1500).
+constexpr float kFaceMax = 0x1p17f;
 
 // Whether gravity and the depth floor are in the ranges the bounds here use. Outside them the
 // dense and flat steps take their operator kernels (1536x1500, g = 981: every row by the faces

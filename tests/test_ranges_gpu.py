@@ -199,6 +199,10 @@ def test_no_data_beds_cost_nothing_on_dry_rows():
     assert _costs_at_most(1.15, dict(change=half(-3.4e38)), usual)
 
 
+def test_lifted_terrain_costs_no_second_evaluation():
+    assert _costs_at_most(1.3, dict(change=lambda q, z: (q, z + 20000.0)), {})
+
+
 @pytest.mark.parametrize("cfg", [dict(g=981.0), dict(h_min=1e-8), dict(h_min_cfl=2.0)])
 def test_physics_outside_the_ranges_costs_the_operators(cfg):
     assert _costs_at_most(1.5, cfg, {})
