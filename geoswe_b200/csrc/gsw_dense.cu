@@ -6,18 +6,21 @@
 
 namespace gsw {
 
-// Standalone wave speed of the current state over the interior (lammax_fp32_lean): a thread
+// Standalone wave speed of the current state over the interior (lammax_fp32_lean): a lane
 // per column, four rows of loads in flight, no division of a cell index (8192^2: 0.43 ms with
-// one, of a 0.12 ms copy's worth of bytes).
+// one, of a 0.12 ms copy's worth of bytes). A block's warps lie side by side over the columns, or,
+// on a grid narrower than they are together, `1 << wshift` of them side by side and the others on
+// the next rows (narrow grids left them idle: a step of 200000x12 728 us where 609 are enough).
 template <typename T>
-__global__ void __launch_bounds__(256) dense_lammax_kernel(DenseK<T> p, unsigned long long* out) {
+__global__ void __launch_bounds__(256) dense_lammax_kernel(DenseK<T> p, unsigned long long* out, int wshift) {
     chain_begin();
     const int nx = p.nxp - 2 * p.ngh, ny = p.nyp - 2 * p.ngh;
     unsigned long long lam = 0ull;
-    const int iy = (blockIdx.x * blockDim.y + threadIdx.y) * 32 + threadIdx.x;
+    const int iy = (int)(((blockIdx.x << wshift) + (threadIdx.y & ((1u << wshift) - 1u))) * 32 + threadIdx.x);
+    const int rows = 8 >> wshift, step = (int)gridDim.y * rows;
     if (iy < ny) {
 #pragma unroll 4
-        for (int ix = blockIdx.y; ix < nx; ix += (int)gridDim.y) {
+        for (int ix = blockIdx.y * rows + (threadIdx.y >> wshift); ix < nx; ix += step) {
             const int64_t o = (int64_t)(ix + p.ngh) * p.pitch + (iy + p.ngh);
             const T h = p.q0[o], hu = p.q1[o], hv = p.q2[o];
             const unsigned long long lb = lam_dense_bits(h, hu, hv, p.g, p.h_cfl);
@@ -189,9 +192,12 @@ static int launch_lammax(const GswDenseArgs* a, uint64_t* out, cudaStream_t s) {
     if (rc) return rc;
     if (!out) return set_error(GSW_ERR_INVALID, "lammax: null output");
     const int nx = k.nxp - 2 * k.ngh, ny = k.nyp - 2 * k.ngh;
-    const unsigned gx = (unsigned)((ny + 255) / 256);
-    const unsigned gy = (unsigned)std::min<int64_t>((nx + 3) / 4, std::max<int64_t>(1, 8LL * sm_count() / gx));
-    launch_chained(dense_lammax_kernel<T>, dim3(gx, std::min(gy, 65535u)), dim3(32, 8), s, k, (unsigned long long*)out);
+    int wshift = 0;
+    while (wshift < 3 && (32 << wshift) < ny) ++wshift;
+    const int cols = 32 << wshift, rows = 8 >> wshift;
+    const unsigned gx = (unsigned)((ny + cols - 1) / cols);
+    const unsigned gy = (unsigned)std::min<int64_t>((nx + 4 * rows - 1) / (4 * rows), std::max<int64_t>(1, 8LL * sm_count() / gx));
+    launch_chained(dense_lammax_kernel<T>, dim3(gx, std::min(gy, 65535u)), dim3(32, 8), s, k, (unsigned long long*)out, wshift);
     return check_launch("dense_lammax");
 }
 

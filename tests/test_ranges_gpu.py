@@ -211,3 +211,48 @@ def test_physics_outside_the_ranges_costs_the_operators(cfg):
 @pytest.mark.parametrize("fs,bound", [(dict(g=981.0), 1.6), (dict(h_min=1e-8), 1.6), (dict(h_min=1e-7), 1.2)])
 def test_compressed_physics_outside_the_ranges_costs_the_operators(fs, bound):
     assert _costs_at_most(bound, dict(flat=True, fs=fs), dict(flat=True))
+
+
+def test_wave_speed_of_a_narrow_grid():
+    """The standalone wave speed of a grid a few cells wide keeps its warps busy: its cells take
+    at most eight times as long as those of a wide grid (24 of 32 lanes have no cell)."""
+    from geoswe_b200 import _lib as L
+    from geoswe_b200.solver import _stream
+    times = []
+    for nx, ny in ((1 << 20, 8), (2896, 2896)):
+        q0 = torch.rand((3, nx, ny), device="cuda") + 0.1
+        s = _solver(q0, torch.zeros((nx, ny), device="cuda"), cls=False)
+        a = s._dense_args(s._buf[0], s._buf[1], s._tables())
+        bits = torch.zeros(1, dtype=torch.int64, device="cuda")
+        best = 1e30
+        for _ in range(6):
+            bits.zero_()
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            L.call("gsw_dense_lammax", C.byref(a), C.c_void_p(bits.data_ptr()), _stream())
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        h, hu, hv = s.q_interior
+        want = torch.maximum((hu / h).abs(), (hv / h).abs()) + (9.81 * h).sqrt()
+        got = bits.view(torch.float64).item()
+        assert abs(got - float(want.max())) <= 4e-7 * got      # two roundings more or less
+        times.append(best)
+        del s, q0
+    assert times[0] < 8.0 * times[1]
+
+
+@pytest.mark.parametrize("nx,ny", [(7, 1), (70, 31), (70, 33), (130, 65), (9, 129), (33, 257), (40, 700)])
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_wave_speed_matches_oracle(nx, ny, dtype):
+    """Widths on both sides of each split of a block's warps between columns and rows."""
+    from geoswe_b200 import Config, Mesh2D, Solver2D
+    rng = np.random.default_rng(nx * ny)
+    q0 = np.stack([rng.random((nx, ny)), *rng.standard_normal((2, nx, ny))]).astype(dtype)
+    for at in ((0, 0), (nx - 1, ny - 1), (nx - 1, 0), (nx // 2, ny // 2)):
+        q = q0.copy()
+        q[1][at] = 900.0 * q[0][at]
+        s = Solver2D(Mesh2D(nx=nx, ny=ny, dx=2.0, dy=2.0, ngh=2), Config(dtype=dtype, h_min=1e-6, h_min_cfl=1e-6), q,
+                     np.zeros((nx, ny)))
+        o = oracle.OracleSolver2D(*pad_state(q, np.zeros((nx, ny)), 2, np.dtype(dtype)), 2, 2.0, 2.0, h_min=1e-6)
+        assert s.cfl_dt() == o.cfl_dt()
