@@ -48,41 +48,43 @@ __device__ __forceinline__ int bc_src(int kind, int g, int n, int ngh) {
 
 // blockIdx.y is the ghost row (over every column, corners included) or, from 2 ngh on, the ghost
 // column (over the interior rows), so no thread divides a cell index: a step of a small grid
-// waits for this kernel.
+// waits for this kernel. Halos of more layers than a grid has rows of blocks take several each.
 template <typename T>
 __global__ void bc_fill_kernel(T* q0, T* q1, T* q2, int nxp, int nyp, int ngh, int64_t pitch,
                                int kxm, int kxp, int kym, int kyp, const GswLoopState* st) {
     chain_begin();
     if (st != nullptr && st->done) return;
-    const bool rows = (int)blockIdx.y < 2 * ngh;
-    const int layer = rows ? blockIdx.y : blockIdx.y - 2 * ngh;
-    const bool low = layer < ngh;
-    const int ghost = low ? layer : (rows ? nxp : nyp) - 2 * ngh + layer;
-    const int lo = rows ? 0 : ngh, hi = rows ? nyp : nxp - ngh;
-    for (int along = lo + blockIdx.x * blockDim.x + threadIdx.x; along < hi; along += gridDim.x * blockDim.x) {
-        const int gi = rows ? ghost : along, gj = rows ? along : ghost;
-        const int kx = !rows ? GSW_BC_NONE : low ? kxm : kxp;
-        const bool corner = rows && (gj < ngh || gj >= nyp - ngh);
-        const int ky = rows && !corner ? GSW_BC_NONE : gj < ngh ? kym : kyp;
-        if (kx == GSW_BC_NONE && ky == GSW_BC_NONE) continue;
-        // value of the x pass at (row gi, column cj)
-        auto xval = [&](int cj, T& a, T& u, T& v) {
-            if (kx == GSW_BC_FALL) { a = (T)0; u = (T)0; v = (T)0; return; }
-            const int64_t o = (int64_t)(kx == GSW_BC_NONE ? gi : bc_src(kx, gi, nxp, ngh)) * pitch + cj;
-            a = q0[o]; u = q1[o]; v = q2[o];
-            if (kx == GSW_BC_WALL) u = -u;
-        };
-        T a, u, v;
-        if (ky == GSW_BC_NONE) {                   // a ghost row, or a corner left to the x pass
-            xval(gj, a, u, v);
-        } else if (ky == GSW_BC_FALL) {
-            a = (T)0; u = (T)0; v = (T)0;
-        } else {
-            xval(bc_src(ky, gj, nyp, ngh), a, u, v);
-            if (ky == GSW_BC_WALL) v = -v;
+    for (int64_t edge = blockIdx.y; edge < 4LL * ngh; edge += gridDim.y) {
+        const bool rows = edge < 2LL * ngh;
+        const int layer = (int)(rows ? edge : edge - 2LL * ngh);
+        const bool low = layer < ngh;
+        const int ghost = low ? layer : (rows ? nxp : nyp) - 2 * ngh + layer;
+        const int lo = rows ? 0 : ngh, hi = rows ? nyp : nxp - ngh;
+        for (int along = lo + blockIdx.x * blockDim.x + threadIdx.x; along < hi; along += gridDim.x * blockDim.x) {
+            const int gi = rows ? ghost : along, gj = rows ? along : ghost;
+            const int kx = !rows ? GSW_BC_NONE : low ? kxm : kxp;
+            const bool corner = rows && (gj < ngh || gj >= nyp - ngh);
+            const int ky = rows && !corner ? GSW_BC_NONE : gj < ngh ? kym : kyp;
+            if (kx == GSW_BC_NONE && ky == GSW_BC_NONE) continue;
+            // value of the x pass at (row gi, column cj)
+            auto xval = [&](int cj, T& a, T& u, T& v) {
+                if (kx == GSW_BC_FALL) { a = (T)0; u = (T)0; v = (T)0; return; }
+                const int64_t o = (int64_t)(kx == GSW_BC_NONE ? gi : bc_src(kx, gi, nxp, ngh)) * pitch + cj;
+                a = q0[o]; u = q1[o]; v = q2[o];
+                if (kx == GSW_BC_WALL) u = -u;
+            };
+            T a, u, v;
+            if (ky == GSW_BC_NONE) {                   // a ghost row, or a corner left to the x pass
+                xval(gj, a, u, v);
+            } else if (ky == GSW_BC_FALL) {
+                a = (T)0; u = (T)0; v = (T)0;
+            } else {
+                xval(bc_src(ky, gj, nyp, ngh), a, u, v);
+                if (ky == GSW_BC_WALL) v = -v;
+            }
+            const int64_t go = (int64_t)gi * pitch + gj;
+            q0[go] = a; q1[go] = u; q2[go] = v;
         }
-        const int64_t go = (int64_t)gi * pitch + gj;
-        q0[go] = a; q1[go] = u; q2[go] = v;
     }
 }
 
@@ -214,8 +216,7 @@ extern "C" int gsw_bc_fill(const GswBcArgs* a, void* stream) {
         return set_error(GSW_ERR_INVALID, "bc: bad extents");
     for (int f = 0; f < 4; ++f)
         if (a->kinds[f] < 0 || a->kinds[f] > GSW_BC_NONE) return set_error(GSW_ERR_INVALID, "bc: bad kind %d", a->kinds[f]);
-    if (a->ngh > 16383) return set_error(GSW_ERR_INVALID, "bc: ngh is too large");
-    const dim3 grid((unsigned)std::min((std::max(a->nxp, a->nyp) + 255) / 256, 64), (unsigned)(4 * a->ngh));
+    const dim3 grid((unsigned)std::min((std::max(a->nxp, a->nyp) + 255) / 256, 64), (unsigned)std::min<int64_t>(4LL * a->ngh, 65535));
     cudaStream_t s = (cudaStream_t)stream;
     if (a->dtype == GSW_F32)
         launch_chained(bc_fill_kernel<float>, grid, dim3(256), s, (float*)a->q0, (float*)a->q1, (float*)a->q2, a->nxp, a->nyp,

@@ -256,3 +256,30 @@ def test_wave_speed_matches_oracle(nx, ny, dtype):
                      np.zeros((nx, ny)))
         o = oracle.OracleSolver2D(*pad_state(q, np.zeros((nx, ny)), 2, np.dtype(dtype)), 2, 2.0, 2.0, h_min=1e-6)
         assert s.cfl_dt() == o.cfl_dt()
+
+
+def test_ghost_fill_of_a_deep_halo():
+    """More ghost layers than a launch has rows of blocks (13 GB)."""
+    from geoswe_b200 import _lib as L
+    from geoswe_b200.solver import _ptr, _stream
+    n, ngh = 5, 16390
+    free, _ = torch.cuda.mem_get_info()
+    w = n + 2 * ngh
+    if free < 5 * 4 * w * w:
+        pytest.skip("needs 21 GB of free device memory")
+    inner = torch.rand((n, n), device="cuda")
+    a = L.GswBcArgs()
+    a.abi_version, a.dtype, a.nxp, a.nyp, a.ngh, a.pitch = L.ABI_VERSION, L.F32, w, w, ngh, w
+    q = [torch.zeros((w, w), device="cuda") for _ in range(3)]
+    for x in q:
+        x[ngh:-ngh, ngh:-ngh] = inner
+    a.q0, a.q1, a.q2 = (_ptr(x) for x in q)
+    for f in range(4):
+        a.kinds[f] = L.BC_EXTRAPOLATE
+    L.call("gsw_bc_fill", C.byref(a), _stream())
+    rows = torch.arange(w, device="cuda").sub(ngh).clamp(0, n - 1)
+    for lo in range(0, w, 4096):
+        r = rows[lo:lo + 4096]
+        want = inner[r][:, rows]
+        for x in q:
+            assert torch.equal(x[lo:lo + 4096], want), lo
