@@ -33,6 +33,13 @@ constexpr bool kRefPowBuild = true;
 
 using gsw_rt::set_error;
 using gsw_rt::check_launch;
+// The step kernels index slots, and cells within a tile of rows, by 32-bit integers up to this
+// bound and by 64-bit ones (or the operators, on longer rows) above it. A build with a lower one
+// takes the kernels above it on small meshes, which is how they are tested.
+#ifndef GSW_INDEX32_MAX
+#define GSW_INDEX32_MAX INT32_MAX
+#endif
+
 using gsw_rt::sm_count;
 using gsw_rt::count_launch;
 using gsw_rt::div_const_recip;

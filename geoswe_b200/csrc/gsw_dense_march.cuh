@@ -415,8 +415,8 @@ inline int fill_dense(const GswDenseArgs* a, DenseK<T>& k, bool step) {
     }
     // dense_rows_kernel's offsets within a tile (rows -2 .. tile_rows + 1) are 32-bit
     const int64_t widest = std::max(k.pitch, k.ncls ? k.cpitch : (int64_t)1);
-    k.long_rows = INT32_MAX / widest < 5;
-    if (!k.long_rows) k.tile_rows = (int)std::min<int64_t>(k.tile_rows, INT32_MAX / widest - 4);
+    k.long_rows = GSW_INDEX32_MAX / widest < 5;
+    if (!k.long_rows) k.tile_rows = (int)std::min<int64_t>(k.tile_rows, GSW_INDEX32_MAX / widest - 4);
     if (step) {
         if (!a->state) return set_error(GSW_ERR_INVALID, "dense step: state (GswLoopState*) is required");
         if (a->rain_kind != GSW_RAIN_NONE && a->rain_kind != GSW_RAIN_UNIFORM && a->rain_kind != GSW_RAIN_GRIDDED)

@@ -166,22 +166,24 @@ __global__ void __maxnreg__(REGS) ensemble_step_kernel(GswEnsembleArgs a, FlatMe
     }
 }
 
-// Register caps by GswEnsembleArgs.min_blocks; 64-bit slots where the storage needs them.
-template <bool REFPOW, bool LEAN>
+// Register caps by GswEnsembleArgs.min_blocks.
+template <typename I, bool REFPOW, bool LEAN>
 inline void launch_ensemble_caps(const GswEnsembleArgs* a, const FlatMesh<float>& m, int grid, int W, cudaStream_t st) {
     const dim3 b(32, W);
-    if ((m.nb + 1) * (int64_t)m.bh * GSW_BRICK_PITCH > INT32_MAX)
-        launch_chained(ensemble_step_kernel<int64_t, 128, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
-    else if (a->min_blocks == 3) launch_chained(ensemble_step_kernel<int, 80, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
-    else if (a->min_blocks == 4) launch_chained(ensemble_step_kernel<int, 64, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
-    else if (a->min_blocks == 5) launch_chained(ensemble_step_kernel<int, 72, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
-    else launch_chained(ensemble_step_kernel<int, 96, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
+    if (a->min_blocks == 3) launch_chained(ensemble_step_kernel<I, 80, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
+    else if (a->min_blocks == 4) launch_chained(ensemble_step_kernel<I, 64, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
+    else if (a->min_blocks == 5) launch_chained(ensemble_step_kernel<I, 72, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
+    else launch_chained(ensemble_step_kernel<I, 96, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
 }
 
+// 64-bit slots where the storage needs them.
 template <bool REFPOW>
 inline void launch_ensemble_shape(const GswEnsembleArgs* a, const FlatMesh<float>& m, int grid, int W, cudaStream_t st) {
-    if (a->lean) launch_ensemble_caps<REFPOW, true>(a, m, grid, W, st);
-    else launch_ensemble_caps<REFPOW, false>(a, m, grid, W, st);
+    const bool wide = (m.nb + 1) * (int64_t)m.bh * GSW_BRICK_PITCH > GSW_INDEX32_MAX;
+    if (wide && a->lean) launch_ensemble_caps<int64_t, REFPOW, true>(a, m, grid, W, st);
+    else if (wide) launch_ensemble_caps<int64_t, REFPOW, false>(a, m, grid, W, st);
+    else if (a->lean) launch_ensemble_caps<int, REFPOW, true>(a, m, grid, W, st);
+    else launch_ensemble_caps<int, REFPOW, false>(a, m, grid, W, st);
 }
 
 // Launch of the step over checked arguments (outputs non-null).

@@ -85,30 +85,30 @@ inline int fill_flat(const GswFlatArgs* a, FlatK<T>& k, bool step) {
 }
 
 // Register caps of the binary32 step by GswFlatArgs.min_blocks.
-template <bool STEP, bool REFPOW, bool LEAN>
+template <typename I, bool STEP, bool REFPOW, bool LEAN>
 inline void launch_flat_caps(const FlatK<float>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
     const dim3 b(32, W);
-    if (STEP && mb == 3) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 96 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
-    else if (STEP && mb == 4) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 64 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
-    else if (STEP && mb == 5) launch_chained(flat_march_kernel<float, int, STEP, STEP ? 72 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
-    else launch_chained(flat_march_kernel<float, int, STEP, 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
+    if (STEP && mb == 3) launch_chained(flat_march_kernel<float, I, STEP, STEP ? 96 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
+    else if (STEP && mb == 4) launch_chained(flat_march_kernel<float, I, STEP, STEP ? 64 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
+    else if (STEP && mb == 5) launch_chained(flat_march_kernel<float, I, STEP, STEP ? 72 : 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
+    else launch_chained(flat_march_kernel<float, I, STEP, 80, REFPOW, LEAN, false>, dim3(blocks), b, s, k);
 }
 
 // The production configuration (the LEAN kernel: rain none or uniform, quadratic
-// friction, keep-h, the L2 norm) or the general kernel.
+// friction, keep-h, the L2 norm) or the general kernel; 64-bit slots where the storage needs them.
 template <bool STEP, bool REFPOW>
 inline void launch_flat_shape(const FlatK<float>& k, int mb, unsigned blocks, int W, cudaStream_t s) {
-    const bool lean = k.ph.rain_kind != GSW_RAIN_GRIDDED && k.ph.rain_kind != GSW_RAIN_LOOKUP &&
+    const bool lean = STEP && k.ph.rain_kind != GSW_RAIN_GRIDDED && k.ph.rain_kind != GSW_RAIN_LOOKUP &&
                       k.ph.quad != 0 && k.ph.keep_h != 0 && k.ph.linf == 0;
+    const bool wide = (k.m.nb + 1) * (int64_t)k.m.bh * GSW_BRICK_PITCH > GSW_INDEX32_MAX;
     if (!kFastArith && k.general) {
-        if (STEP && lean)
-            launch_chained(flat_march_kernel<float, int64_t, STEP, 64, REFPOW, STEP, true>, dim3(blocks), dim3(32, W), s, k);
-        else
-            launch_chained(flat_march_kernel<float, int64_t, STEP, 64, REFPOW, false, true>, dim3(blocks), dim3(32, W), s, k);
-    } else if ((k.m.nb + 1) * (int64_t)k.m.bh * GSW_BRICK_PITCH > INT32_MAX)
-        launch_chained(flat_march_kernel<float, int64_t, STEP, 128, REFPOW, false, false>, dim3(blocks), dim3(32, W), s, k);
-    else if (STEP && lean) launch_flat_caps<STEP, REFPOW, STEP>(k, mb, blocks, W, s);
-    else launch_flat_caps<STEP, REFPOW, false>(k, mb, blocks, W, s);
+        if (lean) launch_chained(flat_march_kernel<float, int64_t, STEP, 64, REFPOW, STEP, true>, dim3(blocks), dim3(32, W), s, k);
+        else launch_chained(flat_march_kernel<float, int64_t, STEP, 64, REFPOW, false, true>, dim3(blocks), dim3(32, W), s, k);
+    }
+    else if (wide && lean) launch_flat_caps<int64_t, STEP, REFPOW, STEP>(k, mb, blocks, W, s);
+    else if (wide) launch_flat_caps<int64_t, STEP, REFPOW, false>(k, mb, blocks, W, s);
+    else if (lean) launch_flat_caps<int, STEP, REFPOW, STEP>(k, mb, blocks, W, s);
+    else launch_flat_caps<int, STEP, REFPOW, false>(k, mb, blocks, W, s);
 }
 template <bool STEP, bool REFPOW>
 inline void launch_flat_shape(const FlatK<double>& k, int, unsigned blocks, int W, cudaStream_t s) {
