@@ -45,8 +45,8 @@ def _key(kind, cells):
     except Exception:
         pass
     size = "small" if cells < 1 << 20 else ("medium" if cells < 1 << 24 else "large")
-    # min_blocks names other register caps than in entries without the tag, which are not read
-    return f"{kind}|{dev}|{drv}|{size}|caps 80/96/64/72"
+    # entries timed on other kernels or register caps are without the tag and not read
+    return f"{kind}|{dev}|{drv}|{size}|rows, caps 80/64/48"
 
 
 def load(kind, cells):

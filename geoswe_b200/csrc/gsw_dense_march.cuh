@@ -438,13 +438,15 @@ inline bool lean_config(const DenseK<float>& k) {
            k.ncls != nullptr && k.rain_kind != GSW_RAIN_GRIDDED && k.quad != 0 && k.keep_h != 0;
 }
 
-// Register caps of the binary32 step by GswDenseArgs.min_blocks.
+// Register caps of the binary32 step by GswDenseArgs.min_blocks. 0: 80 registers, or 96 in the
+// fast arithmetic (8192^2 step at 96, 80, 64 registers: 1.716, 1.661 and 1.749 ms exact, 1.181,
+// 1.197 and 1.188 fast).
 template <bool STEP, bool REFPOW, bool LEAN>
 inline void launch_rows_caps(const DenseK<float>& k, int minb, dim3 grid, dim3 block, cudaStream_t s) {
-    if (STEP && minb == 3) launch_chained(dense_rows_kernel<STEP, STEP ? 96 : 80, REFPOW, LEAN>, grid, block, s, k);
+    if (STEP && minb == 3) launch_chained(dense_rows_kernel<STEP, 80, REFPOW, LEAN>, grid, block, s, k);
     else if (STEP && minb == 4) launch_chained(dense_rows_kernel<STEP, STEP ? 64 : 80, REFPOW, LEAN>, grid, block, s, k);
-    else if (STEP && minb == 5) launch_chained(dense_rows_kernel<STEP, STEP ? 72 : 80, REFPOW, LEAN>, grid, block, s, k);
-    else launch_chained(dense_rows_kernel<STEP, 80, REFPOW, LEAN>, grid, block, s, k);
+    else if (STEP && minb == 5) launch_chained(dense_rows_kernel<STEP, STEP ? 48 : 80, REFPOW, LEAN>, grid, block, s, k);
+    else launch_chained(dense_rows_kernel<STEP, STEP && kFastArith ? 96 : 80, REFPOW, LEAN>, grid, block, s, k);
 }
 
 template <bool STEP, bool REFPOW>

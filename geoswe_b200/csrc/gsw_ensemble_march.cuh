@@ -166,13 +166,13 @@ __global__ void __maxnreg__(REGS) ensemble_step_kernel(GswEnsembleArgs a, FlatMe
     }
 }
 
-// Register caps by GswEnsembleArgs.min_blocks.
+// Register caps by GswEnsembleArgs.min_blocks. 0: 96 registers.
 template <typename I, bool REFPOW, bool LEAN>
 inline void launch_ensemble_caps(const GswEnsembleArgs* a, const FlatMesh<float>& m, int grid, int W, cudaStream_t st) {
     const dim3 b(32, W);
     if (a->min_blocks == 3) launch_chained(ensemble_step_kernel<I, 80, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
     else if (a->min_blocks == 4) launch_chained(ensemble_step_kernel<I, 64, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
-    else if (a->min_blocks == 5) launch_chained(ensemble_step_kernel<I, 72, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
+    else if (a->min_blocks == 5) launch_chained(ensemble_step_kernel<I, 48, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
     else launch_chained(ensemble_step_kernel<I, 96, REFPOW, LEAN>, dim3(grid), b, st, *a, m);
 }
 

@@ -176,7 +176,7 @@ typedef struct GswDenseArgs {
     int32_t  tile_rows;        /* rows per warp strip; 0: the largest of 32, 16, 8, 4 that gives at least
                                   twice the warps the GPU runs at once */
     int32_t  warps;            /* warps per block (0: default 4) */
-    int32_t  min_blocks;       /* fp32 step register cap: 0 (80 regs), 3 (96 regs), 4 (64 regs) or 5 (72 regs) */
+    int32_t  min_blocks;       /* fp32 step register cap: 0 (the library's choice), 3 (80 regs), 4 (64 regs) or 5 (48 regs) */
     int32_t  arith;            /* GSW_ARITH_EXACT (default), GSW_ARITH_PORTABLE, or GSW_ARITH_FAST (GSW_F32 step only) */
     /* Window of the cells computed: rows [row_lo, row_hi) x columns [col_lo, col_hi) of
      * the padded grid, inside the usual range (rows and columns [ngh, n - ngh) for the
@@ -286,7 +286,7 @@ typedef struct GswFlatArgs {
     int32_t  dtype;            /* GSW_F32 or GSW_F64: q*, qn*, bed, rain, n_tab and max_h */
     int32_t  brick_h;          /* rows per brick (>= 2) */
     int32_t  warps;            /* warps per block (0: 4) */
-    int32_t  min_blocks;       /* fp32 step register cap: 0 (80 regs), 3 (96 regs), 4 (64 regs) or 5 (72 regs) */
+    int32_t  min_blocks;       /* fp32 step register cap: 0 (the library's choice), 3 (80 regs), 4 (64 regs) or 5 (48 regs) */
     int32_t  arith;            /* GSW_ARITH_EXACT (default), GSW_ARITH_PORTABLE, or GSW_ARITH_FAST (GSW_F32 step only) */
     int64_t  n_bricks;         /* brick n_bricks is the all-zero brick (a missing neighbour) */
     const int32_t* brick_ij;   /* (n_bricks, 2) brick row, brick column */
@@ -512,7 +512,7 @@ typedef struct GswEnsembleArgs {
     int32_t  n_members;
     int32_t  warps;              /* warps per block (0: 4) */
     int32_t  grid;               /* persistent blocks (0: 2 per SM) */
-    int32_t  min_blocks;         /* register cap: 0 (96 regs), 3 (80 regs), 4 (64 regs) or 5 (72 regs) */
+    int32_t  min_blocks;         /* register cap: 0 (the library's choice), 3 (80 regs), 4 (64 regs) or 5 (48 regs) */
     int32_t  arith;              /* GSW_ARITH_EXACT (default), GSW_ARITH_PORTABLE or GSW_ARITH_FAST */
     int32_t  segments;           /* warps per brick: 1, 2 or 4 (as GswFlatArgs.segments), or 0: chosen per
                                     launch from the running members' bricks against the grid's warps */

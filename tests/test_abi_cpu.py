@@ -125,3 +125,22 @@ def test_step_refuses_a_divisor_floor_that_is_not_positive(h_min, h_cfl):
     f.g, f.h_min, f.h_min_cfl = 9.81, h_min, h_cfl
     assert lib.gsw_flat_step(C.byref(f), None) == L.ERR_INVALID
     assert b"must be > 0" in lib.gsw_last_error()
+
+
+def test_register_caps_are_those_the_header_names():
+    """min_blocks of the step kernels keeps its meaning under one ABI version: every launcher
+    gives the values 3, 4 and 5 the register caps the public header names (a default launch
+    that also serves 3 has that cap)."""
+    header = (ROOT / "include" / "gsw.h").read_text()
+    stated = re.findall(r"min_blocks;\s*/\* (?:fp32 step )?register cap: [^*]*?3 \((\d+) regs\), 4 \((\d+) regs\) or 5 \((\d+) regs\)",
+                        header)
+    assert stated == [("80", "64", "48")] * 3                    # dense, flat, ensemble
+    for name in ("gsw_dense_march.cuh", "gsw_flat_march.cuh", "gsw_ensemble_march.cuh"):
+        text = (ROOT / "geoswe_b200" / "csrc" / name).read_text()
+        body = text[text.index("_caps(const"):]
+        body = body[:body.index("\n}\n")]
+        launches = re.findall(r"(?:(?:mb|minb|a->min_blocks) == (\d)\) |else )launch_chained\(\w+<([^>]*)>", body)
+        caps = {}
+        for value, args in launches:
+            caps[value or "other"] = re.findall(r"(?:STEP \? |\b)(48|64|72|80|96)\b", args)[0]
+        assert caps["4"] == "64" and caps["5"] == "48" and caps.get("3", caps["other"]) == "80", (name, caps)
