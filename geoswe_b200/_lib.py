@@ -226,12 +226,15 @@ def lib():
     return L
 
 
-def call(name, *args):
-    L = lib()
-    rc = getattr(L, name)(*args)
+def check(name, rc):
+    """Raise GswError with the status `rc` of entry point `name` unless it is OK."""
     if rc != OK:
-        raise GswError(name, rc, L.gsw_last_error().decode(errors="replace"))
+        raise GswError(name, rc, lib().gsw_last_error().decode(errors="replace"))
     return rc
+
+
+def call(name, *args):
+    return check(name, getattr(lib(), name)(*args))
 
 
 def launch_count() -> int:

@@ -355,8 +355,7 @@ class FlatAdjoint:
 
         def step(k, _keep=keep):
             for fn, a in dirs[k]:
-                if fn(*a) != L.OK:
-                    raise L.GswError(fn.__name__, -1, lib.gsw_last_error().decode(errors="replace"))
+                L.check(fn.__name__, fn(*a))
             self.kernel_launches += n_launch
         return step
 
@@ -545,11 +544,9 @@ class FlatAdjoint:
                 inflow.state = st
             if gauge is not None:
                 gauge.state = st
-            if lib.gsw_dt_finalize(C.byref(p2), C.c_void_p(st), s) != L.OK:
-                raise L.GswError("gsw_dt_finalize", -1, lib.gsw_last_error().decode(errors="replace"))
+            L.check("gsw_dt_finalize", lib.gsw_dt_finalize(C.byref(p2), C.c_void_p(st), s))
             for fn, args in calls:
-                if fn(*args) != L.OK:
-                    raise L.GswError(fn.__name__, -1, lib.gsw_last_error().decode(errors="replace"))
+                L.check(fn.__name__, fn(*args))
             self.kernel_launches += n_launch
             self._lam = [lin, lout]
 

@@ -3,6 +3,7 @@ reversed exactly once, in order N-1 .. 0, from its own state; no more snapshots 
 live than allowed; the forward steps match the binomial optimum."""
 import numpy as np
 import pytest
+import torch
 
 from geoswe_b200.adjoint import Treeverse, binomial_beta, interp_weights, snapshot_chain, treeverse_split
 
@@ -66,3 +67,42 @@ def test_interp_weights_reproduce_numpy():
     fp = rng.normal(size=9)
     t = np.concatenate([rng.uniform(-10, 110, 50), xp])
     assert np.allclose(interp_weights(t, xp) @ fp, np.interp(t, xp, fp), rtol=0, atol=1e-12)
+
+
+@pytest.mark.parametrize("code", [-1, -2, -3, -5])
+@pytest.mark.parametrize("failing", ["gsw_dt_finalize", "gsw_flat_step", "gsw_adj_flat_step"])
+def test_a_failing_launch_keeps_its_status(monkeypatch, failing, code):
+    """The launchers of a recording pass and of a reverse sweep raise GswError with the status
+    the library returned (no GPU: the entry points are stubs)."""
+    from geoswe_b200 import _lib as L
+    from geoswe_b200 import adjoint as A
+
+    class Lib:
+        def __getattr__(self, name):
+            if name == "gsw_last_error":
+                return lambda: b"stub"
+            fn = lambda *a: code if name == failing else L.OK  # noqa: E731
+            fn.__name__ = name
+            return fn
+
+    stub = Lib()
+    monkeypatch.setattr(L, "lib", lambda: stub)
+    monkeypatch.setattr(A, "_stream", lambda: None)
+    monkeypatch.setattr(A, "_ptr", lambda x: None)
+    adj = object.__new__(A.FlatAdjoint)
+    adj.inlet, adj.G, adj.code, adj.adj_min_blocks, adj.kernel_launches = None, 0, L.F32, 8, 0
+    adj.dev, adj._buf, adj._state = torch.device("cpu"), [[None] * 3] * 2, None
+    adj._lam, adj._rbar, adj.n_bar, adj.rate_bar = [[None] * 3, [None] * 3], [None] * 3, None, None
+    adj._state_tab = torch.zeros((2, 128), dtype=torch.uint8)
+    adj._flat_args = lambda *a: L.GswFlatArgs()
+    p = L.GswDtParams()
+    with pytest.raises(L.GswError) as e:
+        if failing == "gsw_adj_flat_step":
+            adj._reverser(p)(0, 0)
+        else:
+            adj._stepper(p, False)(0)
+    assert e.value.code == code and failing in str(e.value)
+    if failing == "gsw_dt_finalize":
+        with pytest.raises(L.GswError) as e:
+            adj._reverser(p)(0, 0)
+        assert e.value.code == code
