@@ -13,6 +13,7 @@ from __future__ import annotations
 import ctypes as C
 import itertools
 import json
+import math
 import os
 from pathlib import Path
 
@@ -44,7 +45,9 @@ def _key(kind, cells):
         drv = str(v.value)
     except Exception:
         pass
-    size = "small" if cells < 1 << 20 else ("medium" if cells < 1 << 24 else "large")
+    # the first two classes: grids on which the dense step's own rule marches one row, or up to three
+    size = next(n for n, top in (("tiny", 1 << 17), ("little", 1 << 19), ("small", 1 << 20), ("medium", 1 << 24),
+                                 ("large", math.inf)) if cells < top)
     # entries timed on other kernels or register caps are without the tag and not read
     return f"{kind}|{dev}|{drv}|{size}|rows, caps 80/64/48"
 

@@ -3,10 +3,12 @@
 // No counterpart in the reference, whose kernels have fixed launch shapes. Each call
 // times the step at every shape of a fixed search space with CUDA events on the
 // caller's stream and buffers, and returns the fastest. The step's outputs serve as
-// scratch; the wave-speed target and the running maximum are left untouched (the
-// timed launches get NULL for both) and the loop state is only read. Results are kept
-// per (device, kernel family, arithmetic, binary size, size class) in a table guarded
-// by a mutex, so a second call for the same class returns without launching.
+// scratch, for the running maximum too where the step keeps one; the wave speed goes to a
+// word of its own. So the timed launches are those of the caller's step (without a wave-speed
+// target they would take another kernel), its target and running maximum stay untouched and the
+// loop state is only read. Results are kept per (device, kernel family, arithmetic, binary
+// size, size class) in a table guarded by a mutex, so a second call for the same class
+// returns without launching.
 #include "gsw_common.cuh"
 #include <map>
 #include <mutex>
@@ -22,7 +24,9 @@ std::map<std::string, GswTuneResult> g_tune_cache;
 std::string tune_key(const char* family, int arith, int dtype, int64_t cells) {
     int dev = -1;
     cudaGetDevice(&dev);
-    const char* size = cells < (1LL << 20) ? "small" : (cells < (1LL << 24) ? "medium" : "large");
+    // the first two classes: grids on which the dense step's own rule marches one row, or up to three
+    const char* size = cells < (1LL << 17) ? "tiny" : cells < (1LL << 19) ? "little" : cells < (1LL << 20) ? "small" :
+                       cells < (1LL << 24) ? "medium" : "large";
     return std::string(family) + "|" + std::to_string(dev) + "|" + std::to_string(arith) + "|" +
            std::to_string(dtype) + "|" + size;
 }
@@ -37,6 +41,18 @@ int check_not_done(const GswLoopState* st, cudaStream_t s) {
     if (h.done) return set_error(GSW_ERR_INVALID, "autotune: the loop state is done; time a live state");
     return GSW_OK;
 }
+
+// Device word of the timed launches' wave speed; zero, and freed with the object.
+struct LamWord {
+    uint64_t* p = nullptr;
+    explicit LamWord(cudaStream_t s) {
+        if (cudaMalloc(&p, sizeof(*p)) != cudaSuccess) { p = nullptr; cudaGetLastError(); return; }
+        cudaMemsetAsync(p, 0, sizeof(*p), s);
+    }
+    ~LamWord() { cudaFree(p); }
+    LamWord(const LamWord&) = delete;
+    LamWord& operator=(const LamWord&) = delete;
+};
 
 // Mean time (ms) of `reps` launches of `launch` after one untimed launch; < 0 if the
 // shape is refused (an invalid combination), which is skipped.
@@ -69,6 +85,8 @@ extern "C" int gsw_dense_autotune(const GswDenseArgs* a, int32_t reps, int32_t u
         if (it != g_tune_cache.end()) { *out = it->second; return GSW_OK; }
     }
     if (int rc = check_not_done(a->state, s)) return rc;
+    const LamWord lam(s);
+    if (!lam.p) return set_error(GSW_ERR_CUDA, "autotune: no device memory for the wave speed");
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
         return set_error(GSW_ERR_CUDA, "autotune: cudaEventCreate failed");
@@ -80,8 +98,8 @@ extern "C" int gsw_dense_autotune(const GswDenseArgs* a, int32_t reps, int32_t u
         for (int w : warps)
             for (int mb : caps) {
                 GswDenseArgs b = *a;
-                b.lam_target = nullptr;
-                b.max_h = nullptr;
+                if (a->lam_target) b.lam_target = lam.p;
+                if (a->max_h) b.max_h = a->qn0;
                 b.tile_rows = tr; b.warps = w; b.min_blocks = mb;
                 const float ms = time_shape([&] { return gsw_dense_step(&b, stream); }, reps, s, e0, e1);
                 if (ms < 0.0f) continue;
@@ -113,6 +131,8 @@ extern "C" int gsw_flat_autotune(const GswFlatArgs* a, int32_t reps, int32_t use
         if (it != g_tune_cache.end()) { *out = it->second; return GSW_OK; }
     }
     if (int rc = check_not_done(a->state, s)) return rc;
+    const LamWord lam(s);
+    if (!lam.p) return set_error(GSW_ERR_CUDA, "autotune: no device memory for the wave speed");
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
         return set_error(GSW_ERR_CUDA, "autotune: cudaEventCreate failed");
@@ -125,8 +145,8 @@ extern "C" int gsw_flat_autotune(const GswFlatArgs* a, int32_t reps, int32_t use
             for (int g : segs) {
                 if (g > 0 && a->brick_h % g != 0) continue;
                 GswFlatArgs b = *a;
-                b.lam_target = nullptr;
-                b.max_h = nullptr;
+                if (a->lam_target) b.lam_target = lam.p;
+                if (a->max_h) b.max_h = a->qn0;
                 b.warps = w; b.min_blocks = mb; b.segments = g;
                 const float ms = time_shape([&] { return gsw_flat_step(&b, stream); }, reps, s, e0, e1);
                 if (ms < 0.0f) continue;

@@ -601,10 +601,11 @@ GSW_API int gsw_loop_commit(GswLoopState* state, void* stream);
 /*          register cap min_blocks {0, 3, 4, 5}                               */
 /*   flat:  warps {2, 4, 8} x min_blocks {0, 3, 4, 5} x segments {0, 1, 2, 4}   */
 /* The step's outputs (qn*) are overwritten; lam_target and max_h are not      */
-/* touched; the loop state is read (it must not be done). Results are cached   */
-/* per device, kernel family, arithmetic, dtype and size class (< 2^20,        */
-/* < 2^24, larger) behind a mutex; use_cache = 1 returns a cached result       */
-/* without launching.                                                          */
+/* touched (the timed steps reduce into scratch where the caller's would reduce */
+/* into them); the loop state is read (it must not be done). Results are cached */
+/* per device, kernel family, arithmetic, dtype and size class (< 2^17, < 2^19, */
+/* < 2^20, < 2^24, larger) behind a mutex; use_cache = 1 returns a cached      */
+/* result without launching.                                                   */
 /* ------------------------------------------------------------------------- */
 typedef struct GswTuneResult {
     uint32_t abi_version;      /* GSW_ABI_VERSION, set by the caller (the rest is written by the library) */

@@ -133,3 +133,36 @@ def test_library_flat_autotune():
     state.copy_(torch.frombuffer(bytearray(bytes(done) + bytes(128 - C.sizeof(done))), dtype=torch.uint8))
     with pytest.raises(L.GswError):
         L.call("gsw_flat_autotune", C.byref(a), 2, 0, C.byref(res), _stream())
+
+
+def test_library_tuner_leaves_the_callers_reductions():
+    """The timed launches reduce a wave speed and keep a running maximum as the caller's step
+    does, in scratch of the tuner's and in the step's outputs: the caller's own stay as they
+    are, on a dense and on a compressed mesh."""
+    from geoswe_b200 import _lib as L
+    from geoswe_b200.solver import _ptr, _stream
+    s, cs = _dense(), _flat()
+    s.run(t_end=1e9, max_steps=6)
+    cs.run(t_end=1e9, max_steps=6)
+    st = L.GswLoopState()
+    st.dt, st.dt_f32 = 0.01, float(np.float32(0.01))
+    state = torch.zeros(128, dtype=torch.uint8, device=s.device)
+    state.copy_(torch.frombuffer(bytearray(bytes(st) + bytes(128 - C.sizeof(st))), dtype=torch.uint8))
+    out, flat_out = torch.empty_like(s._buf[0]), [torch.empty_like(x) for x in cs._q[0]]
+    for name, top, a in (("dense", s._max_h, s._dense_args(s._buf[s._cur], out, s._tables())),
+                         ("flat", cs._max_h, cs._args(cs._q[cs._cur], flat_out))):
+        lam = torch.full((1,), 7, dtype=torch.int64, device=s.device)
+        kept = top.clone()
+        a.state, a.lam_target, a.max_h = _ptr(state), _ptr(lam), _ptr(top)
+        res = L.GswTuneResult()
+        res.abi_version = L.ABI_VERSION
+        L.call(f"gsw_{name}_autotune", C.byref(a), 2, 0, C.byref(res), _stream())
+        torch.cuda.synchronize()
+        assert res.ms > 0 and int(lam) == 7 and torch.equal(top, kept), name
+
+
+def test_size_classes_follow_the_automatic_shape():
+    """A shape tuned on one grid is not read back for one whose automatic shape differs."""
+    from geoswe_b200 import autotune
+    keys = [autotune._key("dense", n * n) for n in (96, 512, 777, 2048, 8192)]
+    assert len(set(keys)) == 5
