@@ -73,7 +73,7 @@ __device__ __forceinline__ BrickView brick_view(const FlatMesh<T>& m, int64_t bi
 
 template <typename T>
 __device__ __forceinline__ void load_state(const FlatMesh<T>& m, int64_t s, Cell<T>& c) {
-    c.h = __ldg(m.q0 + s); c.hu = __ldg(m.q1 + s); c.hv = __ldg(m.q2 + s); c.b = __ldg(m.b + s);
+    c.h = ld_state(m.q0 + s); c.hu = ld_state(m.q1 + s); c.hv = ld_state(m.q2 + s); c.b = ld_state(m.b + s);
 }
 
 // ---------------------------------------------------------------------------- A
@@ -103,8 +103,8 @@ struct AdjTailRow {
                 rh = rh + frame[(int64_t)(i - ph.ngh) * ph.ny + (j - ph.ngh)];
             }
             const float h1 = h + dt * rh;
-            const float hu1 = __ldg(m.q1 + o) + dt * rhu;
-            const float hv1 = __ldg(m.q2 + o) + dt * rhv;
+            const float hu1 = ld_state(m.q1 + o) + dt * rhu;
+            const float hv1 = ld_state(m.q2 + o) + dt * rhv;
             const int cls = m.ncls ? (int)m.ncls[o] : 0;
             const float n = ph.ntab[cls];
             const Bar3<float> out_b = load_bar(p.li0, p.li1, p.li2, o);
@@ -160,10 +160,10 @@ __global__ void __launch_bounds__(128, MINB) adj_tail_kernel(AdjK<T> p) {
         const int bh = m.bh;
         const int r0 = seg * bh / p.segs, r1 = (seg + 1) * bh / p.segs;
         Cell<T> cur, nx;
-        const T b_m2 = __ldg(m.b + v.slot(r0 - 2, lane));
+        const T b_m2 = ld_state(m.b + v.slot(r0 - 2, lane));
         load_state(m, v.slot(r0 - 1, lane), cur);
         load_state(m, v.slot(r0, lane), nx);
-        T b_next = __ldg(m.b + v.slot(r0 + 1, lane));
+        T b_next = ld_state(m.b + v.slot(r0 + 1, lane));
         make_prims(cur, ph.h_min);
         make_prims(nx, ph.h_min);
         cur.gx = (T)0.5 * (nx.b - b_m2) * ph.inv_dx;
@@ -176,10 +176,10 @@ __global__ void __launch_bounds__(128, MINB) adj_tail_kernel(AdjK<T> p) {
         for (int r = r0; r < r1; ++r) {
             {
                 const int64_t s = v.slot(r + 1, lane);
-                nx.h = __ldg(m.q0 + s); nx.hu = __ldg(m.q1 + s); nx.hv = __ldg(m.q2 + s);
+                nx.h = ld_state(m.q0 + s); nx.hu = ld_state(m.q1 + s); nx.hv = ld_state(m.q2 + s);
             }
             nx.b = b_next;
-            const T b_p2 = __ldg(m.b + v.slot(r + 2, lane));
+            const T b_p2 = ld_state(m.b + v.slot(r + 2, lane));
             make_prims(nx, ph.h_min);
             nx.gx = (T)0.5 * (b_p2 - cur.b) * ph.inv_dx;
             nx.gy = grad_y_flat<T>(m, ph, v, nx.b, r + 1, lane);
@@ -253,14 +253,14 @@ __global__ void __launch_bounds__(128, MINB) adj_face_kernel(AdjK<T> p) {
     const int bh = m.bh;
     const int r0 = seg * bh / p.segs, r1 = (seg + 1) * bh / p.segs;
     Cell<T> cur, nx;
-    const T b_m2 = __ldg(m.b + v.slot(r0 - 2, lane));
+    const T b_m2 = ld_state(m.b + v.slot(r0 - 2, lane));
     int64_t s = v.slot(r0 - 1, lane);
     load_state(m, s, cur);
     Bar3<T> rb_cur = load_bar<T>(p.rb0, p.rb1, p.rb2, s);
     s = v.slot(r0, lane);
     load_state(m, s, nx);
     Bar3<T> rb_nx = load_bar<T>(p.rb0, p.rb1, p.rb2, s);
-    T b_next = __ldg(m.b + v.slot(r0 + 1, lane));
+    T b_next = ld_state(m.b + v.slot(r0 + 1, lane));
     make_prims(cur, ph.h_min);
     make_prims(nx, ph.h_min);
     cur.gx = (T)0.5 * (nx.b - b_m2) * ph.inv_dx;
@@ -278,10 +278,10 @@ __global__ void __launch_bounds__(128, MINB) adj_face_kernel(AdjK<T> p) {
     rb_cur = rb_nx;
     for (int r = r0; r < r1; ++r) {
         s = v.slot(r + 1, lane);
-        nx.h = __ldg(m.q0 + s); nx.hu = __ldg(m.q1 + s); nx.hv = __ldg(m.q2 + s);
+        nx.h = ld_state(m.q0 + s); nx.hu = ld_state(m.q1 + s); nx.hv = ld_state(m.q2 + s);
         rb_nx = load_bar<T>(p.rb0, p.rb1, p.rb2, s);
         nx.b = b_next;
-        const T b_p2 = __ldg(m.b + v.slot(r + 2, lane));
+        const T b_p2 = ld_state(m.b + v.slot(r + 2, lane));
         make_prims(nx, ph.h_min);
         nx.gx = (T)0.5 * (b_p2 - cur.b) * ph.inv_dx;
         nx.gy = grad_y_flat<T>(m, ph, v, nx.b, r + 1, lane);

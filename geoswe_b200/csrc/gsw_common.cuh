@@ -53,6 +53,13 @@ __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// A load in a chained kernel. Its blocks may start before the kernel ahead has ended, and a
+// read-only load (__ldg) asks for memory that nothing writes while the kernel runs: the compiler
+// may move it, over chain_begin too, and the cache need not see the other kernel's writes. So
+// these are plain loads (of the same speed: 1536x1500 step 79.2 us with either).
+template <typename T>
+__device__ __forceinline__ T ld_state(const T* p) { return *p; }
+
 template <class... P, class... A>
 inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
     cudaLaunchAttribute at[1];

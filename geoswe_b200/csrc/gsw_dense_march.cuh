@@ -46,8 +46,8 @@ struct DenseK {
 };
 
 template <typename T>
-__device__ __forceinline__ T ldg_at(const T* a, int64_t pitch, int i, int j) {
-    return __ldg(a + (int64_t)i * pitch + j);
+__device__ __forceinline__ T ld_at(const T* a, int64_t pitch, int i, int j) {
+    return ld_state(a + (int64_t)i * pitch + j);
 }
 
 // Central y-gradient of the bed at (row, lane column): neighbours come from the
@@ -56,16 +56,16 @@ template <typename T>
 __device__ __forceinline__ T grad_y(const DenseK<T>& p, T bc, int row, int c, int lane) {
     T bl = __shfl_up_sync(0xffffffffu, bc, 1);
     T br = __shfl_down_sync(0xffffffffu, bc, 1);
-    if (lane == 0)  bl = ldg_at(p.b, p.pitch, row, max(c - 1, 0));
-    if (lane == 31) br = ldg_at(p.b, p.pitch, row, min(c + 1, p.nyp - 1));
+    if (lane == 0)  bl = ld_at(p.b, p.pitch, row, max(c - 1, 0));
+    if (lane == 31) br = ld_at(p.b, p.pitch, row, min(c + 1, p.nyp - 1));
     return (T)0.5 * (br - bl) * p.inv_dy;
 }
 
 template <typename T>
 __device__ __forceinline__ void load_cell(const DenseK<T>& p, Cell<T>& c, int row, int col) {
-    c.h = ldg_at(p.q0, p.pitch, row, col);
-    c.hu = ldg_at(p.q1, p.pitch, row, col);
-    c.hv = ldg_at(p.q2, p.pitch, row, col);
+    c.h = ld_at(p.q0, p.pitch, row, col);
+    c.hu = ld_at(p.q1, p.pitch, row, col);
+    c.hv = ld_at(p.q2, p.pitch, row, col);
 }
 
 template <typename T>
@@ -132,17 +132,17 @@ __global__ void __maxnreg__(REGS) dense_march_kernel(DenseK<T> p) {
 
     if (warp_active && i0 < i1) {
         Cell<T> cur, nx;
-        const T b_m2 = ldg_at(p.b, p.pitch, i0 - 2, cl);
+        const T b_m2 = ld_at(p.b, p.pitch, i0 - 2, cl);
         load_cell(p, cur, i0 - 1, cl);
-        cur.b = ldg_at(p.b, p.pitch, i0 - 1, cl);
+        cur.b = ld_at(p.b, p.pitch, i0 - 1, cl);
         load_cell(p, nx, i0, cl);
-        nx.b = ldg_at(p.b, p.pitch, i0, cl);
-        T b_next = ldg_at(p.b, p.pitch, i0 + 1, cl);
+        nx.b = ld_at(p.b, p.pitch, i0, cl);
+        T b_next = ld_at(p.b, p.pitch, i0 + 1, cl);
         // prefetch of the row after next: its loads are in flight during this row's faces
-        T pf_h = ldg_at(p.q0, p.pitch, i0 + 1, cl);
-        T pf_hu = ldg_at(p.q1, p.pitch, i0 + 1, cl);
-        T pf_hv = ldg_at(p.q2, p.pitch, i0 + 1, cl);
-        T pf_b = ldg_at(p.b, p.pitch, i0 + 2, cl);
+        T pf_h = ld_at(p.q0, p.pitch, i0 + 1, cl);
+        T pf_hu = ld_at(p.q1, p.pitch, i0 + 1, cl);
+        T pf_hv = ld_at(p.q2, p.pitch, i0 + 1, cl);
+        T pf_b = ld_at(p.b, p.pitch, i0 + 2, cl);
         make_prims(cur, p.h_min);
         make_prims(nx, p.h_min);
         cur.gx = (T)0.5 * (nx.b - b_m2) * p.inv_dx;
@@ -165,10 +165,10 @@ __global__ void __maxnreg__(REGS) dense_march_kernel(DenseK<T> p) {
             nx.b = b_next;
             const T b_p2 = pf_b;
             if (r + 1 < i1) {           // rows r+2 / r+3 exist: the strip ends at i1 <= nxp - lo
-                pf_h = ldg_at(p.q0, p.pitch, r + 2, cl);
-                pf_hu = ldg_at(p.q1, p.pitch, r + 2, cl);
-                pf_hv = ldg_at(p.q2, p.pitch, r + 2, cl);
-                pf_b = ldg_at(p.b, p.pitch, r + 3, cl);
+                pf_h = ld_at(p.q0, p.pitch, r + 2, cl);
+                pf_hu = ld_at(p.q1, p.pitch, r + 2, cl);
+                pf_hv = ld_at(p.q2, p.pitch, r + 2, cl);
+                pf_b = ld_at(p.b, p.pitch, r + 3, cl);
             }
             make_prims(nx, p.h_min);
             nx.gx = (T)0.5 * (b_p2 - cur.b) * p.inv_dx;
@@ -210,8 +210,8 @@ __global__ void __maxnreg__(REGS) dense_march_kernel(DenseK<T> p) {
                             rr0 = rh + frame[(int64_t)(r - p.ngh) * (p.nyp - 2 * p.ngh) + (c - p.ngh)];
                     }
                     T h = cur.h + dt * rr0;
-                    T hu = ldg_at(p.q1, p.pitch, r, c) + dt * rhu;     // reloaded: not carried down the march
-                    T hv = ldg_at(p.q2, p.pitch, r, c) + dt * rhv;
+                    T hu = ld_at(p.q1, p.pitch, r, c) + dt * rhu;     // reloaded: not carried down the march
+                    T hv = ld_at(p.q2, p.pitch, r, c) + dt * rhv;
                     T n = (T)0;
                     if (LEAN) n = p.ntab[cls_r];
                     else if (p.friction_kind == GSW_FRICTION_TABLE)
@@ -251,10 +251,10 @@ struct DenseRows {
     int pitch, cl, co;           // cl: the lane's column, co: the one beyond the halo column
     __device__ __forceinline__ void state(int k, float& h, float& hu, float& hv) const {
         const int o = k * pitch + cl;
-        h = __ldg(q0 + o); hu = __ldg(q1 + o); hv = __ldg(q2 + o);
+        h = ld_state(q0 + o); hu = ld_state(q1 + o); hv = ld_state(q2 + o);
     }
-    __device__ __forceinline__ float bed(int k) const { return __ldg(b + (k * pitch + cl)); }
-    __device__ __forceinline__ float bed_out(int k) const { return __ldg(b + (k * pitch + co)); }
+    __device__ __forceinline__ float bed(int k) const { return ld_state(b + (k * pitch + cl)); }
+    __device__ __forceinline__ float bed_out(int k) const { return ld_state(b + (k * pitch + co)); }
 };
 
 // A row's update (STEP) or its residual. REFPOW: Manning's h^(-4/3) by powf (GSW_ARITH_EXACT)
@@ -305,8 +305,8 @@ struct DenseRow {
         }
         FState s;
         s.h = h + dt * rh;
-        s.hu = __ldg(p.q1 + base + o) + dt * rhu;     // reloaded: not carried down the march
-        s.hv = __ldg(p.q2 + base + o) + dt * rhv;
+        s.hu = ld_state(p.q1 + base + o) + dt * rhu;     // reloaded: not carried down the march
+        s.hv = ld_state(p.q2 + base + o) + dt * rhv;
         const float n = LEAN ? p.ntab[cls] : manning(r, r * p.pitch + c);
         const bool fric = LEAN || p.friction_kind != GSW_FRICTION_NONE;
         bool slow = (kFastArith && p.general) || (!LEAN && (p.quad == 0 || p.keep_h == 0));

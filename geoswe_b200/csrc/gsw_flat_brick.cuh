@@ -79,8 +79,8 @@ __device__ __forceinline__ T grad_y_flat(const FlatMesh<T>& m, const FlatPhys<T>
                                          int r, int lane) {
     T bl = __shfl_up_sync(0xffffffffu, bc, 1);
     T br = __shfl_down_sync(0xffffffffu, bc, 1);
-    if (lane == 0)  bl = __ldg(m.b + v.outer_b(r, 0));
-    if (lane == 31) br = __ldg(m.b + v.outer_b(r, 31));
+    if (lane == 0)  bl = ld_state(m.b + v.outer_b(r, 0));
+    if (lane == 31) br = ld_state(m.b + v.outer_b(r, 31));
     return (T)0.5 * (br - bl) * ph.inv_dy;
 }
 
@@ -128,12 +128,12 @@ struct FlatRows {
     }
     __device__ __forceinline__ void state(int k, float& h, float& hu, float& hv) const {
         const I s = slot(r0 + k);
-        h = __ldg(m.q0 + s); hu = __ldg(m.q1 + s); hv = __ldg(m.q2 + s);
+        h = ld_state(m.q0 + s); hu = ld_state(m.q1 + s); hv = ld_state(m.q2 + s);
     }
-    __device__ __forceinline__ float bed(int k) const { return __ldg(m.b + slot(r0 + k)); }
+    __device__ __forceinline__ float bed(int k) const { return ld_state(m.b + slot(r0 + k)); }
     __device__ __forceinline__ float bed_out(int k) const {
         const int r = r0 + k;
-        return __ldg(m.b + (r < 0 || r >= bh ? zero : out + (I)(r * GSW_BRICK_PITCH)));
+        return ld_state(m.b + (r < 0 || r >= bh ? zero : out + (I)(r * GSW_BRICK_PITCH)));
     }
 };
 
@@ -190,8 +190,8 @@ struct FlatRow {
         }
         FState s;
         s.h = h;
-        s.hu = __ldg(m.q1 + o);                       // reloaded: not carried down the march
-        s.hv = __ldg(m.q2 + o);
+        s.hu = ld_state(m.q1 + o);                       // reloaded: not carried down the march
+        s.hv = ld_state(m.q2 + o);
         if (active) {
             if (ph.rain_kind == GSW_RAIN_UNIFORM) rh = rh + rate;
             else if (!LEAN && ph.rain_kind == GSW_RAIN_GRIDDED) {
@@ -238,14 +238,14 @@ __device__ __forceinline__ unsigned long long flat_brick_operators(const FlatMes
     uint32_t lam32 = 0u;             // binary32: the L2 norm's key
     const int bh = m.bh;
     Cell<T> cur, nx;
-    const T b_m2 = __ldg(m.b + v.slot(r0 - 2, lane));
-    { const int64_t s = v.slot(r0 - 1, lane); cur.h = __ldg(m.q0 + s); cur.hu = __ldg(m.q1 + s); cur.hv = __ldg(m.q2 + s); cur.b = __ldg(m.b + s); }
-    { const int64_t s = v.slot(r0, lane); nx.h = __ldg(m.q0 + s); nx.hu = __ldg(m.q1 + s); nx.hv = __ldg(m.q2 + s); nx.b = __ldg(m.b + s); }
-    T b_next = __ldg(m.b + v.slot(r0 + 1, lane));
+    const T b_m2 = ld_state(m.b + v.slot(r0 - 2, lane));
+    { const int64_t s = v.slot(r0 - 1, lane); cur.h = ld_state(m.q0 + s); cur.hu = ld_state(m.q1 + s); cur.hv = ld_state(m.q2 + s); cur.b = ld_state(m.b + s); }
+    { const int64_t s = v.slot(r0, lane); nx.h = ld_state(m.q0 + s); nx.hu = ld_state(m.q1 + s); nx.hv = ld_state(m.q2 + s); nx.b = ld_state(m.b + s); }
+    T b_next = ld_state(m.b + v.slot(r0 + 1, lane));
     // prefetch of the row after next (rows up to bh+1 exist: the brick below or the zero brick)
     int64_t sp = v.slot(r0 + 1, lane);
-    T pf_h = __ldg(m.q0 + sp), pf_hu = __ldg(m.q1 + sp), pf_hv = __ldg(m.q2 + sp);
-    T pf_b = __ldg(m.b + v.slot(r0 + 2, lane));
+    T pf_h = ld_state(m.q0 + sp), pf_hu = ld_state(m.q1 + sp), pf_hv = ld_state(m.q2 + sp);
+    T pf_b = ld_state(m.b + v.slot(r0 + 2, lane));
     make_prims(cur, ph.h_min);
     make_prims(nx, ph.h_min);
     cur.gx = (T)0.5 * (nx.b - b_m2) * ph.inv_dx;
@@ -270,8 +270,8 @@ __device__ __forceinline__ unsigned long long flat_brick_operators(const FlatMes
         const T b_p2 = pf_b;
         if (r + 1 < r1) {
             sp = v.slot(r + 2, lane);
-            pf_h = __ldg(m.q0 + sp); pf_hu = __ldg(m.q1 + sp); pf_hv = __ldg(m.q2 + sp);
-            pf_b = __ldg(m.b + v.slot(r + 3, lane));
+            pf_h = ld_state(m.q0 + sp); pf_hu = ld_state(m.q1 + sp); pf_hv = ld_state(m.q2 + sp);
+            pf_b = ld_state(m.b + v.slot(r + 3, lane));
         }
         make_prims(nx, ph.h_min);
         nx.gx = (T)0.5 * (b_p2 - cur.b) * ph.inv_dx;
@@ -306,7 +306,7 @@ __device__ __forceinline__ unsigned long long flat_brick_operators(const FlatMes
                     if (!active) { rh = (T)0; rhu = (T)0; rhv = (T)0; }
                     m.o0[o] = rh; m.o1[o] = rhu; m.o2[o] = rhv;
                 } else if (!active) {
-                    m.o0[o] = cur.h; m.o1[o] = __ldg(m.q1 + o); m.o2[o] = __ldg(m.q2 + o);
+                    m.o0[o] = cur.h; m.o1[o] = ld_state(m.q1 + o); m.o2[o] = ld_state(m.q2 + o);
                     if (m.max_h != nullptr && cur.h > (LEAN ? mh_r : m.max_h[o])) m.max_h[o] = cur.h;
                 } else {
                     T rr0 = rh;
@@ -318,8 +318,8 @@ __device__ __forceinline__ unsigned long long flat_brick_operators(const FlatMes
                         rr0 = rr0 + frame[ph.lookup[o]];
                     }
                     T h = cur.h + dt * rr0;
-                    T hu = __ldg(m.q1 + o) + dt * rhu;       // reloaded: not carried down the march
-                    T hv = __ldg(m.q2 + o) + dt * rhv;
+                    T hu = ld_state(m.q1 + o) + dt * rhu;       // reloaded: not carried down the march
+                    T hv = ld_state(m.q2 + o) + dt * rhv;
                     const T n = m.ncls ? ph.ntab[LEAN ? cls_r : m.ncls[o]] : ph.ntab[0];
                     wetdry_friction<T>(h, hu, hv, true, n, dt, ph.g, ph.h_min, ph.vcap,
                                        LEAN || ph.quad != 0, LEAN || ph.keep_h != 0, REFPOW);

@@ -144,3 +144,11 @@ def test_register_caps_are_those_the_header_names():
         for value, args in launches:
             caps[value or "other"] = re.findall(r"(?:STEP \? |\b)(48|64|72|80|96)\b", args)[0]
         assert caps["4"] == "64" and caps["5"] == "48" and caps.get("3", caps["other"]) == "80", (name, caps)
+
+
+def test_chained_kernels_use_no_read_only_loads():
+    """Kernels launched as programmatic dependents may run while the kernel before them still
+    writes: __ldg, which asks for memory unwritten during the kernel, is not for them."""
+    for path in sorted((ROOT / "geoswe_b200" / "csrc").glob("*.cu*")):
+        code = "\n".join(line.split("//")[0] for line in path.read_text().splitlines())
+        assert "__ldg" not in code and "ld.global.nc" not in code and "__restrict__" not in code, path.name
