@@ -29,7 +29,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", *EXACT, "-lineinfo", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-fvisibility=hidden", "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr"]
 # The fast-arithmetic compilation of the binary32 step kernels (gsw_fast.cu): FMA
 # contraction and flush-to-zero; its square root and division are the approximate
-# instructions named in gsw_core.cuh.
+# forms named in gsw_core.cuh and gsw_face.cuh.
 FAST_SOURCES = {"gsw_fast.cu"}
 FAST_FLAGS = ["--fmad=true", "-ftz=true"] + [f for f in NVCC_FLAGS if f not in EXACT]
 

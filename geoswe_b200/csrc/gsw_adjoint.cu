@@ -436,7 +436,8 @@ static int fill_adj(const GswFlatAdjArgs* a, AdjK<T>& k) {
     ph.rain_kind = f.rain_kind; ph.rain = (const T*)f.rain; ph.ngh = f.ngh; ph.nx = f.nx; ph.ny = f.ny;
     ph.ntab = (const T*)f.n_tab;
     ph.lookup = f.rain_lookup; ph.ncol = f.rain_ncol;
-    ph.g_recip = (T)0;          // the recomputed faces divide (the same bits as the forward's)
+    ph.g_recip = (T)0;          // no check of g's reciprocal: binary64 faces divide, binary32 ones
+                                // take rcp_in(g) (face_phys); the same bits as the forward's
     ph.ref_pow = f.arith == GSW_ARITH_EXACT ? 1 : 0;
     k.st = f.state;
     k.li0 = (const T*)a->lam_in0; k.li1 = (const T*)a->lam_in1; k.li2 = (const T*)a->lam_in2;

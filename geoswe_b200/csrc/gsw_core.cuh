@@ -131,7 +131,9 @@ __device__ __forceinline__ float div_znz<float>(float a, float b) {
 // Fast arithmetic (gsw_fast.cu, compiled with FMA contraction and flush-to-zero):
 // binary32 square root and division by the hardware approximations, sqrt.approx
 // (relative error about 2^-23) and div.full (at most 2 ulp, full range); no slow path,
-// so no zero guards. Binary64 keeps the IEEE operations.
+// so no zero guards. They serve the operator forms (the standalone wave speed, the friction's
+// power and limiter, steps outside the usual options); the step's own faces and update take
+// the coarser products of gsw_face.cuh. Binary64 keeps the IEEE operations.
 __device__ __forceinline__ float gsqrt(float a) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));

@@ -190,8 +190,8 @@ inline void launch_ensemble_shape(const GswEnsembleArgs* a, const FlatMesh<float
 inline int launch_ensemble_step(const GswEnsembleArgs* a, cudaStream_t st) {
     const int W = a->warps > 0 ? a->warps : 4;
     if (W < 1 || W > 8) return set_error(GSW_ERR_INVALID, "ensemble: warps must be in [1, 8]");
-    // 16 warps per SM: what the registers leave room for (8 of them idled half the issue slots:
-    // a step of eight members, 0.9 M cells, 73.7 us against 55.7 us)
+    // 16 warps per SM, what the registers leave room for (a step of eight members, 0.68 M active
+    // cells, with 8, 16 and 24 of them: 73.2, 57.9 and 56.3 us)
     const int grid = a->grid > 0 ? a->grid : std::max(1, 16 / W) * sm_count();
     const int S = a->segments > 0 ? a->segments : 1;
     if ((S != 1 && S != 2 && S != 4) || a->brick_h % S != 0 || a->segments < 0)

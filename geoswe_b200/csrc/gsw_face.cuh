@@ -1,11 +1,11 @@
 // gsw_face.cuh -- the binary32 faces and update of the step kernels, without the IEEE
 // division and square-root operators, and the column march that drives them.
 //
-// The step is bound by instruction issue (83 % of the issue slots, 13 % of the DRAM bandwidth at
-// 4096^2). With the operators it takes 30.8 warp instructions per cell, of which their
-// sequences, range tests and branches around their slow paths are a third; without them 25.1,
-// and 17.6 in the fast arithmetic (20.3 before): 4096^2 step 0.538 -> 0.453 ms and 0.360 ->
-// 0.317 ms, the compressed mesh (2.5 M active cells) 0.132 -> 0.097 ms and 0.089 -> 0.072 ms.
+// The step is bound by instruction issue (4096^2: 83 % of the issue slots, 16 % of the peak DRAM
+// throughput). With the operators it takes 30.8 warp instructions per cell, of which their
+// sequences, range tests and branches around their slow paths are a third; without them 24.5,
+// and 17.5 in the fast arithmetic (20.3 before): 4096^2 step 0.538 -> 0.436 ms and 0.360 ->
+// 0.310 ms, the compressed mesh (4096^2, 60 % active) 0.602 -> 0.449 ms and 0.399 -> 0.331 ms.
 // Here the roots and quotients are the bare sequences:
 //   * sqrt(x): y = rsqrt.approx(x), g = RN(x y), d = x - g g (one FMA, exact),
 //     RN(g + d (y / 2)): Newton's correction with the exact residual (P. Markstein, "IA-64 and
@@ -26,12 +26,15 @@
 //
 // Two faces (or two rows) at a time in packed arithmetic (add/mul.rn.f32x2) was measured and
 // is no faster: pairing the operands costs moves (21.0 and 22.4 instructions per cell, where
-// the unpaired face takes 25.1), and 100 to 128 registers leave half the resident warps
-// (4096^2 step 0.472 and 0.459 ms). ptxas also fuses a packed product into a packed sum, with
+// the unpaired face took 25.1), and 100 to 128 registers leave half the resident warps
+// (4096^2 step 0.472 and 0.459 ms, unpaired 0.453). ptxas also fuses a packed product into a packed sum, with
 // --fmad=false too.
 //
-// In the fast arithmetic (GSW_FAST_ARITH) roots and divisions are the approximate ones and
-// nothing is flagged.
+// In the fast arithmetic (GSW_FAST_ARITH) a root is x rsqrt.approx(x) and a quotient a rcp.approx(b),
+// each within 2^-22 of the exact value; nothing is flagged, and divisors of 2^126 and more give 0
+// and an infinite operand of a root NaN. The wave speed that sets dt is taken the same way. The
+// depth error against binary64 after 16 steps on 3000x4096 is 8.2e-7 where sqrt.approx and
+// div.full gave 8.1e-7.
 #pragma once
 #include "gsw_core.cuh"
 
@@ -88,14 +91,14 @@ __device__ __forceinline__ uint32_t min3(uint32_t a, uint32_t b, uint32_t c) { r
 // cell's |h| + |b| + |u| + |v|, a face's depths are at most 4 M, its wave speeds under 4 M (under 8 M
 // from a velocity), the star speed's denominator under 2^6 M^2 = 2^40 and its numerator under
 // 2^8 M^3 = 2^59, so that every quotient of a numerator above 2^-80 is a normal number and its
-// residual exact. 2^17 leaves the usual no-data values (-9999,
-// -32768, 99999) and elevations in feet or centimetres to these faces: at 2^14, terrain lifted by
-// 20000 took 145 us per step where 81 is enough (1536x1500).
+// residual exact. 2^17 leaves the usual no-data values (-9999, -32768, 99999) and elevations in
+// feet or centimetres to these faces: at 2^14, terrain lifted by 20000 took 145 us per step where
+// 86 is enough (1536x1500).
 constexpr float kFaceMax = 0x1p17f;
 
 // Whether gravity and the depth floor are in the ranges the bounds here use. Outside them the
 // dense and flat steps take their operator kernels (1536x1500, g = 981: every row by the faces
-// here and then again by the operators took 149 us where the operators alone take 111).
+// here and then again by the operators took 148 us where the operators alone take 100).
 __host__ __device__ inline bool face_ranges(float g, float h_min) {
     return g >= 1.0f && g <= 128.0f && h_min >= 0x1p-24f && h_min <= 1.0f;
 }
@@ -269,13 +272,15 @@ static __device__ __noinline__ void update_general(FState& s, bool friction, flo
 
 // wetdry_friction (quadratic friction, keep-h) and the wave speed of the new state in one:
 // the reciprocal of the depth is shared by the friction's velocities and the wave speed's.
-// FLAT: the flat loop's L2 speed (h_cfl == h_min there), else the dense loop's maximum norm.
+// FLAT: the flat loop's L2 speed of a cell that h_min_cfl does not floor (h_cfl is h_min there),
+// else the dense loop's maximum norm.
 // Returns whether a value is outside the proven ranges (s is then unchanged and
 // update_general has to be used): non-finite or large values, a nonzero squared speed under
 // 2^-100, a speed above vcap (its limiter divides again), a friction number above 2^100. A
 // momentum under 2^-100 needs no test: its velocity is under 2^-76 whatever its last bits, and
 // its square rounds to 0. Neither do the wave speed's own root and quotient: where one is not
-// exact it is below 2^-48 and absorbed by sqrt(g h) >= 2^-12.
+// exact it is below 2^-48 and absorbed by sqrt(g h) >= 2^-12, or, in a dense cell between h_cfl
+// and h_min, its momentum is 0 and g h at least 2^-90 by the host's test of h_cfl.
 template <bool FLAT, bool REFPOW>
 __device__ __forceinline__ bool update_in(FState& s, bool friction, float n, float dt, float g, float h_min, float vcap,
                                           float h_cfl) {

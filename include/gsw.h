@@ -174,8 +174,10 @@ typedef struct GswDenseArgs {
     const uint8_t* cfl_skip;   /* interior (nx, ny) C-order: 1 = excluded from the wave speed */
     double   h_cfl;            /* wave-speed wet threshold (and divisor), > 0; h_min > 0 too */
     int32_t  tile_rows;        /* rows per warp strip; 0: the largest of 32, 16, 8, 4 that gives at least
-                                  twice the warps the GPU runs at once */
-    int32_t  warps;            /* warps per block (0: default 4) */
+                                  twice the warps the GPU runs at once, and on grids with under four rows
+                                  for each of those, the fewest rows (1 to 4) that they cover at once */
+    int32_t  warps;            /* warps per block (0: 4; fp32 with fewer warps than three times those the
+                                  GPU runs at once: 2) */
     int32_t  min_blocks;       /* fp32 step register cap: 0 (the library's choice), 3 (80 regs), 4 (64 regs) or 5 (48 regs) */
     int32_t  arith;            /* GSW_ARITH_EXACT (default), GSW_ARITH_PORTABLE, or GSW_ARITH_FAST (GSW_F32 step only) */
     /* Window of the cells computed: rows [row_lo, row_hi) x columns [col_lo, col_hi) of
@@ -511,7 +513,7 @@ typedef struct GswEnsembleArgs {
     int64_t  n_bricks;           /* bricks of all members; brick n_bricks is the zero brick */
     int32_t  n_members;
     int32_t  warps;              /* warps per block (0: 4) */
-    int32_t  grid;               /* persistent blocks (0: 2 per SM) */
+    int32_t  grid;               /* persistent blocks (0: 16 warps' worth per SM, at least one) */
     int32_t  min_blocks;         /* register cap: 0 (the library's choice), 3 (80 regs), 4 (64 regs) or 5 (48 regs) */
     int32_t  arith;              /* GSW_ARITH_EXACT (default), GSW_ARITH_PORTABLE or GSW_ARITH_FAST */
     int32_t  segments;           /* warps per brick: 1, 2 or 4 (as GswFlatArgs.segments), or 0: chosen per

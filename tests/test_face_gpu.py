@@ -2,7 +2,7 @@
 
 Their roots and quotients are compared with the operators over the ranges they are used in;
 states outside those ranges (non-finite values, tiny and subnormal momenta and depths, beds
-and depths above 2^14, depth floors and gravity outside face_ranges) with the C oracle, bit for
+and depths above 2^17, depth floors and gravity outside face_ranges) with the C oracle, bit for
 bit, since they take the scalar operators instead. The portable arithmetic: a CPU cannot
 reproduce CUDA's powf.
 """
