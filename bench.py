@@ -204,8 +204,10 @@ def counters():
 
 
 def _traffic(kind, cells):
+    """DRAM bytes per launch by the kernel's capture, and where they are from; nothing for a capture of
+    other sources than the running build's."""
     c = counters().get(kind)
-    if not c or c.get("dram_bytes_per_cell") is None:
+    if not c or c.get("dram_bytes_per_cell") is None or not c["current_build"]:
         return None, None
     return (c["dram_bytes_per_cell"] * cells / 1e9,
             {"unit": "GB per launch", "source": f"profiles/counters.json[{kind}] ({c.get('workload')})",
@@ -216,10 +218,11 @@ def _traffic(kind, cells):
 def issue_roofline(kind, cells, kern_ms, clocks):
     """Issue-rate roofline of a step kernel: achieved warp instructions per second (the
     ncu count per cell x cells / the CUDA-event launch time) against 4 x SMs x the
-    sampled SM clock (max clock when no sample)."""
+    sampled SM clock (max clock when no sample). None when the count was captured on other
+    sources than the running build's: it would be that of another kernel."""
     import torch
     c = counters().get(kind)
-    if not c or c.get("warp_inst_per_cell") is None:
+    if not c or c.get("warp_inst_per_cell") is None or not c["current_build"]:
         return None
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
     mhz = (clocks or {}).get("sm_mhz") or (clocks or {}).get("sm_max_mhz") or 1965.0
@@ -290,7 +293,7 @@ def measure_dense(args, z, cls, n, world, arith="exact"):
     torch.cuda.nvtx.range_push("kernel_timing")        # the launches an ncu capture targets
     kern_ms = time_step_kernel(s, reps=args.kernel_reps)
     torch.cuda.nvtx.range_pop()
-    shape = {"tile_rows": s._tile_rows or "auto", "warps": s._warps or 4, "min_blocks": s._min_blocks}
+    shape = {"tile_rows": s._tile_rows or "auto", "warps": s._warps or "auto", "min_blocks": s._min_blocks}
     del s
     torch.cuda.empty_cache()
     if world > 1:
