@@ -14,12 +14,23 @@ import pytest
 
 import oracle
 from tests._cases import pad_state, same
-from tests.test_face_gpu import KINDS, extreme_state
+from tests.test_face_gpu import KINDS as _KINDS
+from tests.test_face_gpu import extreme_state as _extreme_state
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 NTAB = np.array([0.02, 0.05, 0.09], np.float32)
+KINDS = _KINDS + ["vast"]
+
+
+def extreme_state(kind, nx, ny, seed):
+    """As test_face_gpu's; "vast" is its "huge" with depths, beds and momenta eight times larger, which
+    are then beyond the limit of the faces (2^17)."""
+    if kind != "vast":
+        return _extreme_state(kind, nx, ny, seed)
+    q0, bed = _extreme_state("huge", nx, ny, seed)
+    return q0 * np.float32(8.0), bed * np.float32(8.0)
 
 
 def _classes(nx, ny, seed):
@@ -53,6 +64,13 @@ def _same_runs(q0, bed, steps=4, **phys):
 
 
 # ------------------------------------------------------------------- the production kernels
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("g,h_min", [(9.81, 1e-6), (981.0, 1e-6), (9.81, 1e-8)])
+def test_extreme_states_with_a_class_table(kind, g, h_min):
+    q0, bed = extreme_state(kind, 61, 64, seed=7)
+    _same_runs(q0, bed, g=g, h_min=h_min)
+
+
 def _compressed(q0, bed, fs=None, **cfg):
     from geoswe_b200.compressed import CompressedSolver
     nx, ny = bed.shape
@@ -92,6 +110,69 @@ def test_wave_speed_floor_of_the_dense_step(h_min_cfl):
     s, o = _solver(q0, bed, h_min_cfl=h_min_cfl), _oracle(q0, bed, h_cfl=h_min_cfl)
     assert s.run(1e9, max_steps=4) == o.run(1e9, max_steps=4)
     assert s.t == o.t and same(s.q_interior.cpu().numpy(), o.q[:, 2:-2, 2:-2])
+
+
+@pytest.mark.parametrize("arith", ["portable", "exact"])
+def test_extreme_members_equal_their_own_runs(arith):
+    """Every kind of state, gravity and depth floor in one ensemble."""
+    from geoswe_b200.ensemble import Ensemble
+    specs = [(k, fs) for k in KINDS for fs in ({}, dict(g=981.0), dict(h_min=1e-7))]
+
+    def member(k, i):
+        return _compressed(*extreme_state(specs[k][0], 61, 67, seed=20 + i), specs[k][1], arith=arith)
+
+    alone = [member(k, k) for k in range(len(specs))]
+    ens = Ensemble([member(k, k) for k in range(len(specs))])
+    assert ens.lean
+    n = [cs.run(1e9, max_steps=5) for cs in alone]
+    assert ens.run(1e9, max_steps=5) == n
+    for k, cs in enumerate(alone):
+        assert ens.members[k].t == cs.t, specs[k]
+        for c in range(3):
+            assert same(ens.flat(k, c).cpu().numpy(), cs.flat(c).cpu().numpy()), (specs[k], c)
+
+
+@pytest.mark.parametrize("kind", ["huge", "vast", "still", "moving", "nodata"])
+def test_adjoint_rows_equal_the_operators(kind):
+    """The reverse step's recomputed rows against the operators: with gravity times 2^8, speeds
+    times 2^4 and times over 2^4, every operation of the step scales by a power of two, so depths
+    and their adjoints are the same bits and the momenta's scale, but gravity is then outside
+    the faces' range and every row goes through the operators."""
+    from geoswe_b200.adjoint import FlatAdjoint
+    N, out, dts = 3, [], None
+    for up in (1.0, 16.0):
+        q0, bed = extreme_state(kind if kind in ("huge", "vast") else "still", 61, 67, seed=4)
+        if kind == "moving":
+            q0[1:] = q0[0] * np.random.default_rng(6).standard_normal(q0[1:].shape).astype(np.float32)
+        if kind == "nodata":
+            bed[:, 30:50] = 1.0e6
+            q0[:, :, 26:54] = 0.0
+        q0[1:] *= np.float32(up)
+        cs = _compressed(q0, bed, dict(g=9.81 * up * up))
+        cs.vcap = 1.0e12                              # the limiter's 1e-10 does not scale
+        act = np.nonzero(cs.is_active != 0)[0]
+        adj = FlatAdjoint(cs, gauges=act[::97], n_steps=N, window=N, snapshots=2, rain_times=np.array([0.0]),
+                          rain_base=np.array([1e-5 * up]))
+        adj.set_params(NTAB / up, 1.0)
+        adj.forward()
+        if dts is None:
+            dts = adj.dt_tab.clone()
+        adj.dt_tab.copy_(dts / up)                    # the rule's 1e-12 does not scale either
+        adj._t_tab = np.concatenate([[0.0], np.cumsum(dts[:N].cpu().numpy() / up)])
+        adj._build_state_table()
+        series = adj.forward(replay=True).cpu().numpy()
+        gn, gs, _ = adj.gradients(np.zeros_like(series) + 0.1)
+        lam = [adj.adjoint_state(c)[cs._slot].cpu().numpy() * np.float32(1.0 if c == 0 else up) for c in range(3)]
+        lam = [np.where(np.abs(x) < 2.0 ** -100, np.float32(0.0), x) for x in lam]
+        out.append((series, gn.cpu().numpy() / up, gs, lam))
+    (s0, n0, r0, l0), (s1, n1, r1, l1) = out
+    assert same(s0, s1)
+    assert np.abs(l0[0]).max() > 0
+    for c in range(3):
+        assert same(l0[c], l1[c]), c
+    # sums over atomics in any order: binary64 rounding of at most 61 * 67 * 3 terms each
+    assert np.abs(n0 - n1).max() <= 1e-12 * np.abs(n0).max() + 1e-300
+    assert abs(r0 - r1) <= 1e-12 * abs(r0)
 
 
 # ---------------------------------------------------------------------------- no-data beds
