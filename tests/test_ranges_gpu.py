@@ -3,8 +3,10 @@ against the C oracle or another path, bit for bit, in the kernels of the product
 (a class table on the dense mesh, the L2 wave speed on the compressed one, the ensemble, the
 adjoint), and what they cost, as a ratio of two times of the same kernels on one GPU.
 
-Each bound on a ratio lies between what the operators alone cost (at most 1.3 of the ordinary
-step) and what evaluating every row twice did (1.4 to 1.9).
+Each bound on a ratio lies between what is measured (no-data beds 1.00 of the ordinary step,
+lifted terrain 1.10, the operators alone 1.28 on the dense mesh and 1.41 on the compressed one,
+films under the wave speed's floor 1.03) and what evaluating rows twice cost (1.39, 1.83, 1.86,
+1.93, 1.86).
 """
 import ctypes as C
 import functools
@@ -104,10 +106,10 @@ def test_extreme_states_on_the_compressed_mesh_with_the_l2_speed(kind, fs):
         assert same(cs.flat(c).cpu().numpy(), o.q[c]), c
 
 
-@pytest.mark.parametrize("h_min_cfl", [1e-3, 2.0])
-def test_wave_speed_floor_of_the_dense_step(h_min_cfl):
+@pytest.mark.parametrize("h_min,h_min_cfl", [(1e-6, 1e-3), (1e-6, 2.0), (1e-3, 1e-6)])
+def test_wave_speed_floor_of_the_dense_step(h_min, h_min_cfl):
     q0, bed = extreme_state("film", 61, 64, seed=2)
-    s, o = _solver(q0, bed, h_min_cfl=h_min_cfl), _oracle(q0, bed, h_cfl=h_min_cfl)
+    s, o = _solver(q0, bed, h_min=h_min, h_min_cfl=h_min_cfl), _oracle(q0, bed, h_min=h_min, h_cfl=h_min_cfl)
     assert s.run(1e9, max_steps=4) == o.run(1e9, max_steps=4)
     assert s.t == o.t and same(s.q_interior.cpu().numpy(), o.q[:, 2:-2, 2:-2])
 
